@@ -383,15 +383,6 @@ void launch_force_eval(tmd_system *s, float scale, bool want_vatom) {
   prof_begin(s);
   launch_descriptor(d, s->st, s->launches);
   prof_end(s, 1);
-  MlpArgs ma{};
-  ma.nl = m->h.nl; ma.actfn = m->h.actfn; ma.resnet = m->h.resnet; ma.nin = m->h.nin;
-  int maxh = 1;
-  for (int l = 1; l < m->h.nl; l++) maxh = std::max(maxh, m->h.sizes[l]);
-  ma.maxh = maxh; ma.tr = m->mlp_tr; ma.smem = m->mlp_smem; ma.resident = m->mlp_resident;
-  ma.warped = m->mlp_warped;
-  ma.streamed = m->mlp_streamed; ma.stages = m->mlp_stages; ma.status = s->status;
-  ma.ntiles = s->ntiles; ma.tiles = s->tiles; ma.perm = s->perm; ma.G = s->G;
-  ma.dEdG = s->dEdG; ma.E = s->E; ma.layers = m->d_layers;
   prof_begin(s);
   if (m->h.tdnp) {
     TdnpArgs td{};
@@ -424,6 +415,16 @@ void launch_force_eval(tmd_system *s, float scale, bool want_vatom) {
     if (m->tc_fp8) launch_mlp_fp8(ta, s->st, s->launches);
     else launch_mlp_tc(ta, s->st, s->launches);
   } else {
+    const MlpPlan &pl = m->mlp;
+    const MlpPlan::Form &f = pl.form[s->mlp_form];
+    MlpArgs ma{};
+    ma.nl = m->h.nl; ma.actfn = m->h.actfn; ma.resnet = m->h.resnet; ma.nin = m->h.nin;
+    std::copy(m->h.sizes.begin(), m->h.sizes.end(), ma.sizes);
+    ma.nt = pl.nt; ma.form = s->mlp_form; ma.nchunk = pl.nchunk;
+    ma.grid = std::min(s->ntiles, pl.nsm * f.ctas); ma.smem = f.smem;
+    ma.stream = m->d_mlp_stream; ma.scratch = s->mlp_scratch; ma.scratch_f4 = f.scratch_f4;
+    ma.status = s->status; ma.ntiles = s->ntiles; ma.tiles = s->tiles; ma.perm = s->perm;
+    ma.G = s->G; ma.dEdG = s->dEdG; ma.E = s->E; ma.layers = m->d_layers;
     launch_mlp_fp32(ma, s->st, s->launches);
   }
   prof_end(s, 2);
@@ -455,13 +456,44 @@ int map_types(const tmd_model *m, int n, const int *type, std::vector<int> &elem
   return TMD_OK;
 }
 
+int mlp_tiles(tmd_system *s, const int *cnt, std::vector<int> &tiles) {
+  const tmd_model *m = s->m;
+  const int nelt = m->h.nelt;
+  int rows = m->mlp_tr;
+  if (rows == 0) {
+    s->mlp_form = mlp_fp32_form(m->mlp, cnt, nelt);
+    rows = m->mlp.form[s->mlp_form].rows;
+  }
+  tiles.clear();
+  for (int e = 0, start = 0; e < nelt; start += cnt[e], e++)
+    for (int o = 0; o < cnt[e]; o += rows) {
+      tiles.push_back(e);
+      tiles.push_back(start + o);
+      tiles.push_back(std::min(rows, cnt[e] - o));
+    }
+  s->ntiles = (int)tiles.size() / 3;
+  if (m->mlp_tr == 0) {
+    const MlpPlan::Form &f = m->mlp.form[s->mlp_form];
+    const size_t need = (size_t)std::min(s->ntiles, m->mlp.nsm * f.ctas) * f.scratch_f4;
+    if (need > s->mlp_scratch_alloc) {
+      TMD_CUDA(cudaStreamSynchronize(s->st));
+      drop_graph(s);  // captured steps hold the old scratch
+      dfree(s->mlp_scratch);
+      s->mlp_scratch_alloc = 0;
+      TMD_CUDA(dalloc(&s->mlp_scratch, need));
+      s->mlp_scratch_alloc = need;
+    }
+  }
+  return TMD_OK;
+}
+
 int set_elements(tmd_system *s, int n, const int *elem) {
   const HostModel &h = s->m->h;
   s->n = n;
   s->h_elem.assign(elem, elem + n);
   s->nhc_valid = false;  // new atoms: a fresh thermostat
   // atoms grouped by element (TensorMD::calc_tensor_density i2row order),
-  // MLP tiles of up to mlp_tr atoms of one element
+  // MLP tiles of one element each
   // (ghost atoms, the last s->nghost, have no MLP rows)
   const int ne = n - s->nghost;
   std::vector<int> cnt(h.nelt, 0), start(h.nelt + 1, 0);
@@ -470,13 +502,8 @@ int set_elements(tmd_system *s, int n, const int *elem) {
   std::vector<int> perm(n > 0 ? n : 1), fill(start.begin(), start.end() - 1);
   for (int i = 0; i < ne; i++) perm[fill[elem[i]]++] = i;
   std::vector<int> tiles;
-  for (int e = 0; e < h.nelt; e++)
-    for (int o = 0; o < cnt[e]; o += s->m->mlp_tr) {
-      tiles.push_back(e);
-      tiles.push_back(start[e] + o);
-      tiles.push_back(std::min(s->m->mlp_tr, cnt[e] - o));
-    }
-  s->ntiles = (int)tiles.size() / 3;
+  const int rc = mlp_tiles(s, cnt.data(), tiles);
+  if (rc) return rc;
   if (n > 0) {
     TMD_CUDA(cudaMemcpyAsync(s->elem, s->h_elem.data(), n * sizeof(int), cudaMemcpyHostToDevice,
                              s->st));
@@ -848,15 +875,13 @@ int tmd_model_load(const char *coeff_args, int device, tmd_model **out) {
       MlpLayer &L = layers[(size_t)el * h.nl + l];
       L.K = h.sizes[l];
       L.N = h.sizes[l + 1];
-      float *w = nullptr, *b = nullptr;
+      float *b = nullptr;
       double *wd = nullptr, *bd = nullptr;
-      e = up(h.W[el][l], &w);
-      if (e == cudaSuccess && !h.Bs[el][l].empty()) e = up(h.Bs[el][l], &b);
+      if (!h.Bs[el][l].empty()) e = up(h.Bs[el][l], &b);
       if (l == h.nl - 1) {
         if (e == cudaSuccess) e = upd(h.Wout[el], &wd);
         if (e == cudaSuccess && !h.Bout[el].empty()) e = upd(h.Bout[el], &bd);
       }
-      L.W = w;
       L.b = b;
       L.Wd = wd;
       L.bd = bd;
@@ -933,69 +958,29 @@ int tmd_model_load(const char *coeff_args, int device, tmd_model **out) {
     *out = m;
     return TMD_OK;
   }
-  // MLP: with 64-wide hidden layers and no residual layers the warp-tile
-  // form (a warp per 32 atoms, the element's weights in shared memory);
-  // else the resident-weight form (one persistent CTA per SM) when the
-  // element's hidden weights and a tile's activations fit in shared memory
-  // (128-atom tiles, else 64); else the persistent streamed-weight form
-  // (64-atom tiles, weight chunks copied through a stage ring); else, for
-  // residual MLPs, weights staged per chunk by the threads with 64- or
-  // 32-atom tiles
-  size_t s64 = mlp_fp32_smem(h.nl, h.sizes.data(), 64);
-  size_t s32 = mlp_fp32_smem(h.nl, h.sizes.data(), 32);
-  const size_t sres = mlp_fp32r_smem(h.nl, h.sizes.data(), 128);
-  const size_t sres64 = mlp_fp32r_smem(h.nl, h.sizes.data(), 64);
-  int nsm = 0;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device);
-  int wt_warps = 0;
-  size_t swt = 0;
-  for (int nw = 16; nw >= 8 && wt_warps == 0; nw--) {
-    swt = mlp_fp32w_smem(h.nl, h.sizes.data(), h.resnet, nw);
-    if (swt > 0 && swt <= 227 * 1024) wt_warps = nw;
+  if (!mlp_fp32_accepts(h.nl, h.sizes.data(), h.resnet)) {
+    tmd_model_free(m);
+    return fail(TMD_ERR_MODEL, "MLP too wide for the shared-memory tile");
   }
-  if (wt_warps > 0 && nsm > 0) {
-    // 64-wide hidden layers: the warp-tile form, one CTA of wt_warps warps
-    // per SM, tiles of mlp_fp32w_rows() atoms per warp
-    m->mlp_tr = mlp_fp32w_rows() * wt_warps; m->mlp_smem = swt; m->mlp_resident = nsm;
-    m->mlp_warped = wt_warps;
-  } else if (h.nl >= 2 && sres <= 227 * 1024 && nsm > 0) {
-    m->mlp_tr = 128; m->mlp_smem = sres; m->mlp_resident = nsm;
-  } else if (h.nl >= 2 && sres64 <= 227 * 1024 && nsm > 0) {
-    m->mlp_tr = 64; m->mlp_smem = sres64; m->mlp_resident = nsm;
-  } else if (int stages = 0;
-             nsm > 0 && (m->mlp_smem = mlp_fp32s_smem(h.nl, h.sizes.data(), h.resnet, &stages)) > 0) {
-    // weights streamed through shared memory in chunks (64-atom tiles):
-    // pack each hidden layer's W and W^T into the chunk layouts
-    m->mlp_tr = 64; m->mlp_streamed = nsm; m->mlp_stages = stages;
-    for (int el = 0; el < h.nelt && e == cudaSuccess; el++)
-      for (int l = 0; l + 1 < h.nl && e == cudaSuccess; l++) {
-        MlpLayer &Ly = layers[(size_t)el * h.nl + l];
-        std::vector<float> pf, pb;
-        mlp_fp32s_pack(h.W[el][l].data(), h.sizes[l], h.sizes[l + 1], pf, pb);
-        float *df = nullptr, *db = nullptr;
-        e = up(pf, &df);
-        if (e == cudaSuccess) e = up(pb, &db);
-        Ly.Wp = df;
-        Ly.Wtp = db;
-      }
-    if (e == cudaSuccess)
-      e = cudaMemcpy(m->d_layers, layers.data(), layers.size() * sizeof(MlpLayer),
-                     cudaMemcpyHostToDevice);
+  if (h.precision == TMD_PREC_FP32) {
+    int nsm = 0;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device);
+    m->mlp = mlp_fp32_plan(h.nl, h.sizes.data(), h.actfn, h.resnet, nsm);
+    if (m->mlp.form[0].ctas == 0 || nsm <= 0) {
+      tmd_model_free(m);
+      return fail(TMD_ERR_CUDA, "the FP32 MLP kernel does not fit on this device");
+    }
+    std::vector<float> stream, one;
+    for (int el = 0; el < h.nelt; el++) {
+      mlp_fp32_pack(h.nl, h.sizes.data(), m->mlp.nt, h.W[el].data(), one);
+      stream.insert(stream.end(), one.begin(), one.end());
+    }
+    e = up(stream, &m->d_mlp_stream);
     if (e != cudaSuccess) {
       tmd_model_free(m);
       return fail(TMD_ERR_CUDA, std::string("model upload: ") + cudaGetErrorString(e));
     }
-    mlp_fp32s_prepare(m->mlp_smem);
-  } else if (s64 <= 110 * 1024) {
-    m->mlp_tr = 64; m->mlp_smem = s64;
-  } else if (s32 <= 220 * 1024) {
-    m->mlp_tr = 32; m->mlp_smem = s32;
-  } else {
-    tmd_model_free(m);
-    return fail(TMD_ERR_MODEL, "MLP too wide for the shared-memory tile");
   }
-  if (m->mlp_warped > 0) mlp_fp32w_prepare(m->mlp_smem);
-  else if (m->mlp_streamed == 0) mlp_fp32_prepare(m->mlp_tr, m->mlp_smem, m->mlp_resident > 0);
   for (int l = 1; l < h.nl; l++) m->maxh = std::max(m->maxh, h.sizes[l]);
   if (h.precision == TMD_PREC_TF32X3) {
     // 3xTF32 on tcgen05 (streamed form): W as hi = tf32(W) and lo =
@@ -1260,7 +1245,7 @@ int tmd_system_create(const tmd_model *m, int natoms_cap, double skin,
   if (h.tdnp) { A(tdnp_s, N); A(tdnp_a, N); A(tdnp_tot, 2); }
   A(partial, 1024 * 8); A(scal, 8);
   A(flag, 2); A(status, 2);  // flag[0] rebuild pending, flag[1] rebuilds done
-  A(perm, N); A(tiles, 3 * (N / 32 + h.nelt + 1));
+  A(perm, N); A(tiles, 3 * (N / (m->mlp_tr > 0 ? m->mlp_tr : m->mlp.form[0].rows) + h.nelt + 1));
 #undef A
   if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void **>(&s->h_scal), 8 * sizeof(double));
   if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void **>(&s->h_status), 4 * sizeof(int));
@@ -1289,7 +1274,7 @@ void tmd_system_free(tmd_system *s) {
   dfree(s->wv); dfree(s->eatom); dfree(s->vatom); dfree(s->ke); dfree(s->partial);
   dfree(s->scal); dfree(s->flag); dfree(s->status); dfree(s->perm);
   dfree(s->tdnp_s); dfree(s->tdnp_a); dfree(s->tdnp_tot);
-  dfree(s->tiles); dfree(s->thermo_d);
+  dfree(s->tiles); dfree(s->mlp_scratch); dfree(s->thermo_d);
   dfree(s->cbox); dfree(s->cgeom); dfree(s->acell); dfree(s->coff); dfree(s->cell_out);
   dfree(s->cflag);
   dfree(s->nhc); dfree(s->nhc_ke);

@@ -138,6 +138,19 @@ size_t server_bytes_per_atom(const tmd_model *m, int cap) {
   return a;
 }
 
+// Device bytes of the FP32 MLP's tile list and act' scratch for up to `atoms`
+// atoms: the scratch grows with the tiles until every CTA slot has its own.
+size_t server_mlp_bytes(const tmd_model *m, size_t atoms) {
+  if (m->mlp_tr > 0) return 0;
+  size_t most = 0;
+  for (const MlpPlan::Form &f : m->mlp.form) {
+    if (f.ctas == 0) continue;
+    const size_t tiles = std::min(atoms / f.rows + m->h.nelt, (size_t)m->mlp.nsm * f.ctas);
+    most = std::max(most, tiles * f.scratch_f4 * sizeof(float4));
+  }
+  return most + 12 * (atoms / m->mlp.form[0].rows + m->h.nelt + 1);
+}
+
 // Row length (a multiple of 32) a job of n atoms in box volume vol needs.
 int job_cap(const tmd_server *sv, int n, double vol) {
   return (cap_for_density(sv->s, n / vol) + 31) / 32 * 32;
@@ -239,7 +252,7 @@ int relayout(tmd_server *sv, const std::vector<JobP> &next) {
     s->n = 0;
     return TMD_OK;
   }
-  const int B = s->m->h.nelt, tr = s->m->mlp_tr;
+  const int B = s->m->h.nelt;
   std::unordered_map<const Job *, int> old_cell;
   for (size_t c = 0; c < sv->active.size(); c++) old_cell[sv->active[c].get()] = (int)c;
   std::vector<int> coff(C + 1, 0), srcv(C), fresh(C, 0), total(B, 0), selem;
@@ -270,15 +283,11 @@ int relayout(tmd_server *sv, const std::vector<JobP> &next) {
   const int n = coff[C];
   if (n > s->natoms_cap) return fail(TMD_ERR_CAPACITY, "atoms exceed the batch capacity");
   // MLP element grouping (set_elements' order): element e from start[e],
-  // cell by cell; tiles of up to mlp_tr atoms of one element
+  // cell by cell
   std::vector<int> cur(B, 0), estart((size_t)C * B), tiles;
   for (int e = 1; e < B; e++) cur[e] = cur[e - 1] + total[e - 1];
-  for (int e = 0; e < B; e++)
-    for (int o = 0; o < total[e]; o += tr) {
-      tiles.push_back(e);
-      tiles.push_back(cur[e] + o);
-      tiles.push_back(std::min(tr, total[e] - o));
-    }
+  int rc = mlp_tiles(s, total.data(), tiles);
+  if (rc) return rc;
   for (int c = 0; c < C; c++)
     for (int e = 0; e < B; e++) {
       estart[(size_t)c * B + e] = cur[e];
@@ -287,7 +296,7 @@ int relayout(tmd_server *sv, const std::vector<JobP> &next) {
   s->ncells = C;
   s->h_coff = coff;
   s->h_acell.clear();
-  int rc = cells_geometry(s, boxes.data(), pbc.data());
+  rc = cells_geometry(s, boxes.data(), pbc.data());
   if (rc) return rc;
   TMD_CUDA(cudaMemcpyAsync(s->coff, coff.data(), (C + 1) * sizeof(int), cudaMemcpyHostToDevice,
                            s->st));
@@ -328,7 +337,6 @@ int relayout(tmd_server *sv, const std::vector<JobP> &next) {
   launch_srv_perm(C, B, s->coff, s->elem, sv->estart, s->perm, s->st, s->launches);
   TMD_CUDA(cudaGetLastError());
   s->n = n;
-  s->ntiles = (int)tiles.size() / 3;
   s->h_elem.clear();
   s->have_atoms = true;
   s->forces_valid = false;
@@ -638,7 +646,10 @@ int tmd_server_create_bytes(const tmd_model *m, size_t hbm_bytes, double max_den
   const size_t per = server_bytes_per_atom(m, cap);
   const size_t cell_bytes = (size_t)max_cells * 160;  // boxes, geometry, sums, controls
   if (hbm_bytes <= cell_bytes + per) return fail(TMD_ERR_CAPACITY, "HBM budget below one atom");
-  const size_t atoms = (hbm_bytes - cell_bytes) / per;
+  size_t atoms = (hbm_bytes - cell_bytes) / per;
+  const size_t mlp = server_mlp_bytes(m, atoms);
+  if (mlp < hbm_bytes - cell_bytes)
+    atoms = std::max((hbm_bytes - cell_bytes - mlp) / per, (size_t)1);
   if (atoms > (size_t)kMaxAtoms) return fail(TMD_ERR_CAPACITY, "HBM budget beyond the atom index range");
   return server_create(m, (int)atoms, max_cells, skin, steps_per_tick, cap, out);
 }
@@ -649,7 +660,7 @@ int tmd_server_footprint(const tmd_server *sv, size_t *device_bytes, int *max_at
   const int cap = std::max(sv->s->cap, sv->max_cap);
   if (device_bytes)
     *device_bytes = (size_t)sv->max_atoms * server_bytes_per_atom(sv->m, cap) +
-                    (size_t)sv->max_cells * 160;
+                    server_mlp_bytes(sv->m, sv->max_atoms) + (size_t)sv->max_cells * 160;
   if (max_atoms) *max_atoms = sv->max_atoms;
   if (row_length) *row_length = cap;
   return TMD_OK;

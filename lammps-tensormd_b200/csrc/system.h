@@ -36,12 +36,10 @@ struct tmd_model {
   int tc_cps = 1;        // its CTAs per SM
   int maxh = 1;
   double *d_mass = nullptr;     // per element
-  int mlp_tr = 64;
-  size_t mlp_smem = 0;
-  int mlp_resident = 0;    // > 0: resident-weight MLP, persistent grid size
-  int mlp_warped = 0;      // > 0: warp-tile MLP, warps per CTA (grid mlp_resident)
-  int mlp_streamed = 0;    // > 0: streamed-weight FP32 MLP, persistent grid size
-  int mlp_stages = 0;
+  // atoms per tensor-core MLP tile; 0: the FP32 MLP, tiles by atom count
+  int mlp_tr = 0;
+  tmd::MlpPlan mlp{};           // FP32 MLP
+  float *d_mlp_stream = nullptr;  // its packed weights (in d_buf)
   // temperature-dependent model (tdnp = 1): the nets' layers on the device
   tmd::TdnpLayer *d_tdnp = nullptr;
   size_t tdnp_warp_floats = 0;
@@ -93,6 +91,9 @@ struct tmd_system {
   int *flag = nullptr, *status = nullptr;  // status[0] bits, status[1] longest row needed
   int *perm = nullptr, *tiles = nullptr;
   int ntiles = 0;
+  int mlp_form = 0;                 // FP32 MLP form of the current tiles
+  float4 *mlp_scratch = nullptr;    // its act' scratch
+  size_t mlp_scratch_alloc = 0;
   double *thermo_d = nullptr;
   long thermo_alloc = 0;
   // host
@@ -195,6 +196,9 @@ int map_types(const tmd_model *m, int n, const int *type, std::vector<int> &elem
 // Set n atoms' elements: host mirror, device elem[], MLP element grouping
 // (perm, tiles).  Synchronises the stream.
 int set_elements(tmd_system *s, int n, const int *elem);
+// MLP tiles (element, start, count) of atoms grouped by element, cnt[e] of
+// element e; sets ntiles, and the FP32 form and its scratch.
+int mlp_tiles(tmd_system *s, const int *cnt, std::vector<int> &tiles);
 // Multi-cell mode (batch.cpp): device arrays for up to max_cells cells, the
 // cell layout (atoms per cell, concatenated), per-cell boxes.
 int cells_alloc(tmd_system *s, int max_cells);

@@ -37,6 +37,18 @@ __device__ inline void commit(uint64_t *mbar) {
           smem_u32(mbar)));
 }
 
+// Whether the mbarrier phase has completed (one test, no waiting loop).
+__device__ inline bool mbar_test(uint64_t *mbar, uint32_t phase) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(mbar)), "r"(phase)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait for the mbarrier phase; false on timeout (after `limit`
 // clock cycles).
 __device__ inline bool mbar_wait(uint64_t *mbar, uint32_t phase, long long limit = kWaitCycles) {
@@ -63,6 +75,15 @@ __device__ inline void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, u
       "[%3];" ::"r"(dst),
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
+}
+
+__device__ inline void mbar_init(uint64_t *mbar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar)), "r"(count)
+               : "memory");
+}
+
+__device__ inline void mbar_arrive(uint64_t *mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");
 }
 
 // Arrive on `bar` and add `bytes` to the transaction count of its phase.

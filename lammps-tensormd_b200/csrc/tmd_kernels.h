@@ -106,25 +106,32 @@ void launch_descriptor(const DescArgs &a, cudaStream_t st, long &launches);
 // MLP forward + backward over element-grouped tiles.
 struct MlpLayer {
   int K, N;
-  const float *W;  // [K][N] row-major (npz weights_e_l)
   const float *b;  // [N] or nullptr
-  // output layer only: FP64 copies, the atomic energy is formed in FP64
+  // output layer only, in FP64: the atomic energy is formed in FP64
   const double *Wd;
   const double *bd;
-  // streamed-weight form only (hidden layers): W packed [N/128][K][128] and
-  // W^T packed [K/128][N][128] (mlp_fp32s_pack)
-  const float *Wp;
-  const float *Wtp;
+};
+// FP32 MLP: the tile forms of a net (v = 0..3: 1, 2, 4 or 8 row registers
+// per thread) and their launch sizes.
+struct MlpPlan {
+  int nt, actfn, nsm;  // columns of a weight chunk, activation, SMs
+  int nchunk;          // weight chunks of one tile, forward and backward
+  struct Form {
+    int rows;          // atoms per tile
+    int ctas;          // resident CTAs per SM, 0 if the form does not fit
+    size_t smem;       // dynamic shared memory bytes
+    size_t scratch_f4; // act' scratch per CTA (float4)
+  } form[4];
 };
 struct MlpArgs {
-  int nl, actfn, resnet, nin, maxh;
-  int tr;             // atoms per tile (32 or 64 streamed, 64 or 128 resident)
-  size_t smem;        // dynamic shared memory bytes
-  int resident;       // > 0: resident-weight form, persistent grid of this many CTAs
-  int warped;         // > 0: warp-tile form, this many warps per CTA (tiles of 32 per warp)
-  int streamed;       // > 0: streamed-weight form, persistent grid of this many CTAs
-  int stages;         // its weight-chunk stages
-  int *status;        // timeout bit of the streamed form's bounded waits
+  int nl, actfn, resnet, nin;
+  int sizes[kMaxLayers + 1];
+  int nt, form, grid, nchunk;
+  size_t smem;
+  const float *stream;  // packed weights [nelt][nchunk][32][nt] (mlp_fp32_pack)
+  float4 *scratch;      // act' of the CTAs' tiles
+  size_t scratch_f4;    // per CTA
+  int *status;          // timeout bit of the bounded waits
   int ntiles;
   const int *tiles;   // [ntiles][3] = (element, start, count) into perm
   const int *perm;    // atom indices grouped by element
@@ -135,23 +142,15 @@ struct MlpArgs {
   const MlpLayer *layers;  // [nelt][nl] device array
 };
 void launch_mlp_fp32(const MlpArgs &a, cudaStream_t st, long &launches);
-size_t mlp_fp32_smem(int nl, const int *sizes, int tr);
-// Resident-weight form: shared memory per CTA for tiles of tr atoms (128
-// atoms on 512 threads, or 64 on 256 when the wider tile does not fit).
-size_t mlp_fp32r_smem(int nl, const int *sizes, int tr);
-// Warp-tile form (64-wide hidden layers, no residual layers): shared memory
-// per CTA of `warps` warps, 0 if the form does not apply.
-size_t mlp_fp32w_smem(int nl, const int *sizes, int resnet, int warps);
-int mlp_fp32w_rows();  // atoms per warp tile
-void mlp_fp32w_prepare(size_t smem);
-void mlp_fp32_prepare(int tr, size_t smem, bool resident);
-// Streamed-weight form (weights too large for shared memory): dynamic shared
-// memory and weight stages, 0 if unsupported (residual layers, widths not
-// multiples of 32); host packing of one layer's W into its chunk layouts.
-size_t mlp_fp32s_smem(int nl, const int *sizes, int resnet, int *stages);
-void mlp_fp32s_pack(const float *W, int K, int N, std::vector<float> &fwd,
-                    std::vector<float> &bwd);
-void mlp_fp32s_prepare(size_t smem);
+// Whether the net's widths are within the library's limits.
+bool mlp_fp32_accepts(int nl, const int *sizes, int resnet);
+// Forms and launch sizes of a net on the current device.
+MlpPlan mlp_fp32_plan(int nl, const int *sizes, int actfn, int resnet, int nsm);
+// The form for count[e] atoms per element.
+int mlp_fp32_form(const MlpPlan &p, const int *count, int nelt);
+// One element's weights W[l] ([K][N] row-major) as the chunks of a tile.
+void mlp_fp32_pack(int nl, const int *sizes, int nt, const std::vector<float> *W,
+                   std::vector<float> &out);
 
 // Tensor-core (tcgen05) MLP, BF16 operands (TF32 in the 3xTF32 streamed
 // form).  Weights are packed on the host in chunks of the K-major
