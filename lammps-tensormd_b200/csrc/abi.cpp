@@ -1240,7 +1240,7 @@ int tmd_system_create(const tmd_model *m, int natoms_cap, double skin,
   A(image, 3 * N); A(elem, N);
   A(cell_of, N); A(cell_atoms, N);
   A(nraw, N); A(boff, N * (h.nelt + 1)); A(pcnt, N * h.nelt);
-  A(P, N * h.nelt * h.K * h.D); A(G, N * h.nin); A(dEdG, N * h.nin); A(E, N);
+  A(P, N * h.nelt * h.K * basis_count(h.D)); A(G, N * h.nin); A(dEdG, N * h.nin); A(E, N);
   A(wv, 6 * N); A(eatom, N); A(vatom, 6 * N); A(ke, N);
   if (h.tdnp) { A(tdnp_s, N); A(tdnp_a, N); A(tdnp_tot, 2); }
   A(partial, 1024 * 8); A(scal, 8);

@@ -15,8 +15,8 @@
 // positions one chunk ahead, so the gather latency overlaps the arithmetic.
 // Nothing per pair goes to global memory.
 //
-// Output layout: P[n][B][K][D] (kept for the force kernel), then
-// k_invariants forms G[n][B*K*M] (the MLP input rows, m fastest, as
+// Output layout: P[n][B][K][E] over the E = kBasis<D> functions of basis_p
+// (kept for the force kernel), then k_invariants forms G[n][B*K*M] (the MLP input rows, m fastest, as
 // TensorMD::get_G) from P.
 #pragma once
 
@@ -88,12 +88,14 @@ __device__ inline const BoxP &box_of(const BoxP &box, const BoxP *__restrict__ c
   else return box;
 }
 
-// Monomials as FP32 pairs (D2 = ceil(D/2), the last pair padded with 0).
-template <int D, int D2>
+// The functions P is accumulated over (FORCE: Q is evaluated over) as
+// FP32 pairs (D2 = ceil(E/2), the last pair padded with 0).
+template <int D, int D2, bool FORCE = false>
 __device__ inline void moments2(float x, float y, float z, float2 M2[D2]) {
   float M[2 * D2];
-  moments<D>(x, y, z, M);
-  if (D & 1) M[D] = 0.f;
+  if (FORCE) basis_q<D>(x, y, z, M);
+  else basis_p<D>(x, y, z, M);
+  if (kBasis<D> & 1) M[kBasis<D>] = 0.f;
 #pragma unroll
   for (int p = 0; p < D2; p++) M2[p] = make_float2(M[2 * p], M[2 * p + 1]);
 }
@@ -200,6 +202,25 @@ __device__ inline PairGeo load_pair_geo(const float4 *__restrict__ src, int &t) 
   return decode_pair_geo<RK>(__ldg(src), __ldg(src + 1), t);
 }
 
+// P_0 = sum_j H_k, by far the largest of a filter's sums and the one whose
+// rounding reaches G_0 and G_2 together, is summed chunk by chunk: the chunk's
+// sum starts from zero and is folded into p0 at the end of the chunk.  On BCC
+// cells this takes the descriptor's share of the force error from 2.8e-6 (one
+// running sum, 20 monomials) to 1.7e-6.
+template <int F, int N>
+__device__ __forceinline__ void fold_p0(float2 (&acc)[F][N], float (&p0)[F]) {
+#pragma unroll
+  for (int f = 0; f < F; f++) {
+    p0[f] += acc[f][0].x;
+    acc[f][0].x = 0.f;
+  }
+}
+template <int F, int N>
+__device__ __forceinline__ void take_p0(float2 (&acc)[F][N], const float (&p0)[F]) {
+#pragma unroll
+  for (int f = 0; f < F; f++) acc[f][0].x = p0[f];
+}
+
 template <int TPA, int D, int RK, bool MULTI>
 __global__ void __launch_bounds__(kPairThreads, 4)
 k_descriptor(KParams kp, BoxP box, int n, int cap, const double *__restrict__ x,
@@ -208,7 +229,7 @@ k_descriptor(KParams kp, BoxP box, int n, int cap, const double *__restrict__ x,
              float *__restrict__ G, const BoxP *__restrict__ cbox,
              const int *__restrict__ acell, float4 *__restrict__ pdf,
              float4 *__restrict__ pgeo, int *__restrict__ pcnt) {
-  constexpr int D2 = (D + 1) / 2;
+  constexpr int E = kBasis<D>, D2 = (E + 1) / 2;
   __shared__ GeoSlot geo[2 * kPairThreads + kPairThreads];
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   const int a = gt / TPA;
@@ -242,6 +263,7 @@ k_descriptor(KParams kp, BoxP box, int n, int cap, const double *__restrict__ x,
     for (int q = 0; q < 4; q++)
 #pragma unroll
       for (int p = 0; p < D2; p++) acc[q][p] = make_float2(0.f, 0.f);
+    float p0[4] = {0.f, 0.f, 0.f, 0.f};
     pr.begin(x, row, bo[b], bo[b + 1]);
     for (;;) {
       const int cnt = pr.feed(kp, bx, xi, yi, zi, x, row, pdf_row);
@@ -262,12 +284,14 @@ k_descriptor(KParams kp, BoxP box, int n, int cap, const double *__restrict__ x,
         }
       }
       pr.pop(cnt);
+      fold_p0(acc, p0);
     }
+    take_p0(acc, p0);
     if (sub == 0) pcnt[(size_t)a * B + b] = nact - nact0;
-    // P rows of this lane: 4 filters x D values, contiguous (G = T P^2 is
+    // P rows of this lane: 4 filters x E values, contiguous (G = T P^2 is
     // formed by k_invariants)
-    float *Pp = P + (((size_t)a * B + b) * K + k0) * D;
-    if constexpr (D % 2 == 0) {
+    float *Pp = P + (((size_t)a * B + b) * K + k0) * E;
+    if constexpr (E % 2 == 0) {
       float2 *P2 = reinterpret_cast<float2 *>(Pp);
 #pragma unroll
       for (int q = 0; q < 4; q++)
@@ -277,7 +301,7 @@ k_descriptor(KParams kp, BoxP box, int n, int cap, const double *__restrict__ x,
 #pragma unroll
       for (int q = 0; q < 4; q++)
 #pragma unroll
-        for (int d = 0; d < D; d++) Pp[q * D + d] = (d & 1) ? acc[q][d >> 1].y : acc[q][d >> 1].x;
+        for (int d = 0; d < E; d++) Pp[q * E + d] = (d & 1) ? acc[q][d >> 1].y : acc[q][d >> 1].x;
     }
   }
 }
@@ -299,7 +323,7 @@ k_descriptor_w(KParams kp, BoxP box, int n, int cap, const double *__restrict__ 
                const BoxP *__restrict__ cbox,
                const int *__restrict__ acell, float4 *__restrict__ pdf,
                float4 *__restrict__ pgeo, int *__restrict__ pcnt) {
-  constexpr int D4 = (D + 3) / 4 * 4;
+  constexpr int E = kBasis<D>, D4 = (E + 3) / 4 * 4;
   constexpr int M = D == 1 ? 1 : (D == 4 ? 2 : (D == 10 ? 3 : 4));
   constexpr int P2 = D4 / 2;
   __shared__ GeoSlot geo[2 * kPairThreads + kPairThreads / 4];
@@ -329,9 +353,9 @@ k_descriptor_w(KParams kp, BoxP box, int n, int cap, const double *__restrict__ 
   const unsigned live = live_lanes(gt, (long)n * W);
   auto keep_monomials = [&](int idx, const PairGeo &g) {
     float M[D4];
-    moments<D>(g.ux, g.uy, g.uz, M);
+    basis_p<D>(g.ux, g.uy, g.uz, M);
 #pragma unroll
-    for (int d = D; d < D4; d++) M[d] = 0.f;
+    for (int d = E; d < D4; d++) M[d] = 0.f;
     float4 *dst = reinterpret_cast<float4 *>(mr + idx * D4);
 #pragma unroll
     for (int v = 0; v < D4 / 4; v++)
@@ -348,6 +372,7 @@ k_descriptor_w(KParams kp, BoxP box, int n, int cap, const double *__restrict__ 
     for (int f = 0; f < FPL; f++)
 #pragma unroll
       for (int p = 0; p < P2; p++) acc[f][p] = make_float2(0.f, 0.f);
+    float p0[FPL] = {};
     pr.begin(x, row, bo[b], bo[b + 1]);
     for (;;) {
       const int cnt = pr.feed_with(kp, bx, xi, yi, zi, x, row, pdf_row, keep_monomials);
@@ -377,32 +402,30 @@ k_descriptor_w(KParams kp, BoxP box, int n, int cap, const double *__restrict__ 
         }
       }
       pr.pop(cnt);
+      fold_p0(acc, p0);
     }
+    take_p0(acc, p0);
     if (sub == 0) pcnt[(size_t)a * B + b] = nact - nact0;
-    float *Pp = P + (((size_t)a * B + b) * K + kf) * D;
+    float *Pp = P + (((size_t)a * B + b) * K + kf) * E;
     float *Gp = G + (((size_t)a * B + b) * K + kf) * M;
 #pragma unroll
     for (int f = 0; f < FPL; f++) {
-      if constexpr (D % 2 == 0) {
-        float2 *P2p = reinterpret_cast<float2 *>(Pp + f * D);
+      float Av[E];
 #pragma unroll
-        for (int p = 0; p < D / 2; p++) P2p[p] = acc[f][p];
+      for (int d = 0; d < E; d++) Av[d] = (d & 1) ? acc[f][d >> 1].y : acc[f][d >> 1].x;
+      if constexpr (E % 4 == 0) {
+#pragma unroll
+        for (int v = 0; v < E / 4; v++)
+          reinterpret_cast<float4 *>(Pp + f * E)[v] =
+              make_float4(Av[4 * v], Av[4 * v + 1], Av[4 * v + 2], Av[4 * v + 3]);
       } else {
 #pragma unroll
-        for (int d = 0; d < D; d++) Pp[f * D + d] = (d & 1) ? acc[f][d >> 1].y : acc[f][d >> 1].x;
+        for (int d = 0; d < E; d++) Pp[f * E + d] = Av[d];
       }
-      // G row of the filter, in the order of k_invariants
+      float Gv[M];
+      invariants<D, M>(Av, kp.T, Gv);
 #pragma unroll
-      for (int m = 0; m < M; m++) {
-        float s = 0.f;
-#pragma unroll
-        for (int d = 0; d < D; d++) {
-          const float pv = (d & 1) ? acc[f][d >> 1].y : acc[f][d >> 1].x;
-          s = fmaf(kp.T[m * D + d], pv * pv, s);
-        }
-        if (m == 0) s = copysignf(1.f, acc[f][0].x) * sqrtf(s);
-        Gp[f * M + m] = s;
-      }
+      for (int m = 0; m < M; m++) Gp[f * M + m] = Gv[m];
     }
   }
 }
@@ -425,7 +448,7 @@ k_descriptor_w2(KParams kp, BoxP box, int n, int cap, const double *__restrict__
                 const int *__restrict__ acell, float4 *__restrict__ pdf,
                 float4 *__restrict__ pgeo, int *__restrict__ pcnt) {
   constexpr int FL = W / 2;
-  constexpr int D4 = (D + 3) / 4 * 4;
+  constexpr int E = kBasis<D>, D4 = (E + 3) / 4 * 4;
   constexpr int M = D == 1 ? 1 : (D == 4 ? 2 : (D == 10 ? 3 : 4));
   constexpr int P2 = D4 / 2;
   __shared__ GeoSlot geo[2 * kPairThreads + kPairThreads / 4];
@@ -456,9 +479,9 @@ k_descriptor_w2(KParams kp, BoxP box, int n, int cap, const double *__restrict__
   const unsigned live = live_lanes(gt, (long)n * W);
   auto keep_monomials = [&](int idx, const PairGeo &g) {
     float Mv[D4];
-    moments<D>(g.ux, g.uy, g.uz, Mv);
+    basis_p<D>(g.ux, g.uy, g.uz, Mv);
 #pragma unroll
-    for (int d = D; d < D4; d++) Mv[d] = 0.f;
+    for (int d = E; d < D4; d++) Mv[d] = 0.f;
     float4 *dst = reinterpret_cast<float4 *>(mr + idx * D4);
 #pragma unroll
     for (int v = 0; v < D4 / 4; v++)
@@ -475,6 +498,7 @@ k_descriptor_w2(KParams kp, BoxP box, int n, int cap, const double *__restrict__
     for (int f = 0; f < FPL; f++)
 #pragma unroll
       for (int p = 0; p < P2; p++) acc[f][p] = make_float2(0.f, 0.f);
+    float p0[FPL] = {};
     pr.begin(x, row, bo[b], bo[b + 1]);
     for (;;) {
       const int cnt = pr.feed_with(kp, bx, xi, yi, zi, x, row, pdf_row, keep_monomials);
@@ -503,7 +527,9 @@ k_descriptor_w2(KParams kp, BoxP box, int n, int cap, const double *__restrict__
         }
       }
       pr.pop(cnt);
+      fold_p0(acc, p0);
     }
+    take_p0(acc, p0);
     if (sub == 0) pcnt[(size_t)a * B + b] = nact - nact0;
     // P = stream 0 + stream 1 (both streams hold the sum afterwards)
 #pragma unroll
@@ -515,30 +541,27 @@ k_descriptor_w2(KParams kp, BoxP box, int n, int cap, const double *__restrict__
         acc[f][p] = stream == 0 ? make_float2(acc[f][p].x + ox, acc[f][p].y + oy)
                                 : make_float2(ox + acc[f][p].x, oy + acc[f][p].y);
       }
-    float *Pp = P + (((size_t)a * B + b) * K + kf) * D;
+    float *Pp = P + (((size_t)a * B + b) * K + kf) * E;
     float *Gp = G + (((size_t)a * B + b) * K + kf) * M;
 #pragma unroll
     for (int f = 0; f < FPL; f++) {
       if ((f & 1) != stream) continue;  // each stream writes half the filters
-      if constexpr (D % 2 == 0) {
-        float2 *P2p = reinterpret_cast<float2 *>(Pp + f * D);
+      float Av[E];
 #pragma unroll
-        for (int p = 0; p < D / 2; p++) P2p[p] = acc[f][p];
+      for (int d = 0; d < E; d++) Av[d] = (d & 1) ? acc[f][d >> 1].y : acc[f][d >> 1].x;
+      if constexpr (E % 4 == 0) {
+#pragma unroll
+        for (int v = 0; v < E / 4; v++)
+          reinterpret_cast<float4 *>(Pp + f * E)[v] =
+              make_float4(Av[4 * v], Av[4 * v + 1], Av[4 * v + 2], Av[4 * v + 3]);
       } else {
 #pragma unroll
-        for (int d = 0; d < D; d++) Pp[f * D + d] = (d & 1) ? acc[f][d >> 1].y : acc[f][d >> 1].x;
+        for (int d = 0; d < E; d++) Pp[f * E + d] = Av[d];
       }
+      float Gv[M];
+      invariants<D, M>(Av, kp.T, Gv);
 #pragma unroll
-      for (int m = 0; m < M; m++) {
-        float sacc = 0.f;
-#pragma unroll
-        for (int d = 0; d < D; d++) {
-          const float pv = (d & 1) ? acc[f][d >> 1].y : acc[f][d >> 1].x;
-          sacc = fmaf(kp.T[m * D + d], pv * pv, sacc);
-        }
-        if (m == 0) sacc = copysignf(1.f, acc[f][0].x) * sqrtf(sacc);
-        Gp[f * M + m] = sacc;
-      }
+      for (int m = 0; m < M; m++) Gp[f * M + m] = Gv[m];
     }
   }
 }
@@ -635,7 +658,7 @@ template <int W, int FPL, int D, int RK>
 __global__ void __launch_bounds__(kPairThreads, 8)
 k_descriptor_c(KParams kp, int n, int cap, float *__restrict__ P, float *__restrict__ G,
                const float4 *__restrict__ pgeo, const int *__restrict__ pcnt) {
-  constexpr int D4 = (D + 3) / 4 * 4;
+  constexpr int E = kBasis<D>, D4 = (E + 3) / 4 * 4;
   constexpr int M = D == 1 ? 1 : (D == 4 ? 2 : (D == 10 ? 3 : 4));
   constexpr int P2 = D4 / 2;
   constexpr int SL = D4 + 4;  // floats per slot: monomials, then (r, rlo, fc | tq, ti)
@@ -665,6 +688,7 @@ k_descriptor_c(KParams kp, int n, int cap, float *__restrict__ P, float *__restr
     for (int f = 0; f < FPL; f++)
 #pragma unroll
       for (int p = 0; p < P2; p++) acc[f][p] = make_float2(0.f, 0.f);
+    float p0[FPL] = {};
     float4 ga = make_float4(0.f, 0.f, 0.f, 0.f), gb = ga;
     if (sub < np) {
       ga = __ldg(pg_row + 2 * (pos + sub));
@@ -675,9 +699,9 @@ k_descriptor_c(KParams kp, int n, int cap, float *__restrict__ P, float *__restr
       float *slot = sg + (buf * W + sub) * SL;
       if (sub < cnt) {
         float Mv[D4];
-        moments<D>(ga.z, ga.w, gb.x, Mv);
+        basis_p<D>(ga.z, ga.w, gb.x, Mv);
 #pragma unroll
-        for (int d = D; d < D4; d++) Mv[d] = 0.f;
+        for (int d = E; d < D4; d++) Mv[d] = 0.f;
 #pragma unroll
         for (int v = 0; v < D4 / 4; v++)
           reinterpret_cast<float4 *>(slot)[v] =
@@ -725,31 +749,30 @@ k_descriptor_c(KParams kp, int n, int cap, float *__restrict__ P, float *__restr
         }
       }
       buf ^= 1;
+      fold_p0(acc, p0);
     }
+    take_p0(acc, p0);
     pos += np;
-    float *Pp = P + (((size_t)a * B + b) * K + kf) * D;
+    float *Pp = P + (((size_t)a * B + b) * K + kf) * E;
     float *Gp = G + (((size_t)a * B + b) * K + kf) * M;
 #pragma unroll
     for (int f = 0; f < FPL; f++) {
-      if constexpr (D % 2 == 0) {
-        float2 *P2p = reinterpret_cast<float2 *>(Pp + f * D);
+      float Av[E];
 #pragma unroll
-        for (int p = 0; p < D / 2; p++) P2p[p] = acc[f][p];
+      for (int d = 0; d < E; d++) Av[d] = (d & 1) ? acc[f][d >> 1].y : acc[f][d >> 1].x;
+      if constexpr (E % 4 == 0) {
+#pragma unroll
+        for (int v = 0; v < E / 4; v++)
+          reinterpret_cast<float4 *>(Pp + f * E)[v] =
+              make_float4(Av[4 * v], Av[4 * v + 1], Av[4 * v + 2], Av[4 * v + 3]);
       } else {
 #pragma unroll
-        for (int d = 0; d < D; d++) Pp[f * D + d] = (d & 1) ? acc[f][d >> 1].y : acc[f][d >> 1].x;
+        for (int d = 0; d < E; d++) Pp[f * E + d] = Av[d];
       }
+      float Gv[M];
+      invariants<D, M>(Av, kp.T, Gv);
 #pragma unroll
-      for (int m = 0; m < M; m++) {
-        float sacc = 0.f;
-#pragma unroll
-        for (int d = 0; d < D; d++) {
-          const float pv = (d & 1) ? acc[f][d >> 1].y : acc[f][d >> 1].x;
-          sacc = fmaf(kp.T[m * D + d], pv * pv, sacc);
-        }
-        if (m == 0) sacc = copysignf(1.f, acc[f][0].x) * sqrtf(sacc);
-        Gp[f * M + m] = sacc;
-      }
+      for (int m = 0; m < M; m++) Gp[f * M + m] = Gv[m];
     }
   }
 }
@@ -794,40 +817,31 @@ void launch_descriptor_w(const DescArgs &a, cudaStream_t st) {
 #undef TMD_DESCW_ARGS
 }
 
-// G[b,k,m] = sum_d T[m,d] P[b,k,d]^2, G[b,k,0] = sign(P0) sqrt(.)
-// (kernel_1_fused_device, kernel.cu:1028-1061): one thread per output, the D
-// values of the row from L1, coalesced writes in the MLP row layout.
+// G rows from P (the 4-filter form): one thread per row.
 template <int D, int M>
-__global__ void k_invariants(long nout, KParams kp, const float *__restrict__ P,
+__global__ void k_invariants(long nrow, KParams kp, const float *__restrict__ P,
                              float *__restrict__ G) {
-  __shared__ float sT[M * D];  // lanes read different m: no per-lane param index
-  for (int i = threadIdx.x; i < M * D; i += blockDim.x) sT[i] = kp.T[i];
-  __syncthreads();
-  const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nout) return;
-  const long row = e / M;
-  const int m = (int)(e - row * M);
-  const float *p = P + row * D;
-  float s = 0.f;
+  const long row = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (row >= nrow) return;
+  constexpr int E = kBasis<D>;
+  float A[E], Gv[M];
 #pragma unroll
-  for (int d = 0; d < D; d++) {
-    const float pv = __ldg(p + d);
-    s = fmaf(sT[m * D + d], pv * pv, s);
-  }
-  if (m == 0) s = copysignf(1.f, __ldg(p)) * sqrtf(s);
-  G[e] = s;
+  for (int d = 0; d < E; d++) A[d] = __ldg(P + row * E + d);
+  invariants<D, M>(A, kp.T, Gv);
+#pragma unroll
+  for (int m = 0; m < M; m++) G[row * M + m] = Gv[m];
 }
 
 inline void launch_invariants(const DescArgs &a, cudaStream_t st) {
-  const long nout = (long)a.n * a.kp.B * a.kp.K * a.kp.M;
-  if (nout == 0) return;
+  const long nrow = (long)a.n * a.kp.B * a.kp.K;
+  if (nrow == 0) return;
   const int T = 256;
-  const unsigned grid = (unsigned)((nout + T - 1) / T);
+  const unsigned grid = (unsigned)((nrow + T - 1) / T);
   switch (a.kp.D) {
-    case 1: k_invariants<1, 1><<<grid, T, 0, st>>>(nout, a.kp, a.P, a.G); break;
-    case 4: k_invariants<4, 2><<<grid, T, 0, st>>>(nout, a.kp, a.P, a.G); break;
-    case 10: k_invariants<10, 3><<<grid, T, 0, st>>>(nout, a.kp, a.P, a.G); break;
-    default: k_invariants<20, 4><<<grid, T, 0, st>>>(nout, a.kp, a.P, a.G); break;
+    case 1: k_invariants<1, 1><<<grid, T, 0, st>>>(nrow, a.kp, a.P, a.G); break;
+    case 4: k_invariants<4, 2><<<grid, T, 0, st>>>(nrow, a.kp, a.P, a.G); break;
+    case 10: k_invariants<10, 3><<<grid, T, 0, st>>>(nrow, a.kp, a.P, a.G); break;
+    default: k_invariants<20, 4><<<grid, T, 0, st>>>(nrow, a.kp, a.P, a.G); break;
   }
 }
 

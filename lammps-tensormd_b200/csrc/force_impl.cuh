@@ -29,8 +29,7 @@ namespace tmd {
 
 // dE/dG' of one (atom, block, filter) row (kernel2_GPU, kernel.cu:730-848;
 // tensor_ops.cpp:633-674): dE/dG'_m = dE/dG_m for m > 0 and
-// dE/dG'_0 = 0.5 dE/dG_0 / G_0 (0 when |G_0| < 1e-8); then
-// S[k][d] = 2 P[k][d] sum_m T[m][d] dE/dG'_m, m ascending.
+// dE/dG'_0 = 0.5 dE/dG_0 / G_0 (0 when |G_0| < 1e-8); S follows by dedp_row.
 __device__ inline void dedp_row_g(const float *__restrict__ G, const float *__restrict__ dEdG,
                                   size_t row, int M, float gp[4]) {
 #pragma unroll
@@ -38,15 +37,6 @@ __device__ inline void dedp_row_g(const float *__restrict__ G, const float *__re
   const float g0 = __ldg(G + row * M);
   gp[0] = fabsf(g0) < 1e-8f ? 0.f : gp[0] / g0 * 0.5f;
 }
-__device__ inline float dedp_elem(const float gp[4], const float *T, int D, int M, int d,
-                                  float p) {
-  float t = 0.f;
-#pragma unroll
-  for (int m = 0; m < 4; m++)
-    if (m < M) t = fmaf(gp[m], T[m * D + d], t);
-  return 2.f * t * p;
-}
-
 template <int TPA, int D, int RK, bool MULTI>
 __global__ void __launch_bounds__(kPairThreads, 3)
 k_force(KParams kp, BoxP box, int n, int cap, float scale,
@@ -56,7 +46,7 @@ k_force(KParams kp, BoxP box, int n, int cap, float scale,
         const float *__restrict__ dEdG, float4 *__restrict__ pdf,
         double *__restrict__ wv, const BoxP *__restrict__ cbox,
         const int *__restrict__ acell) {
-  constexpr int D2 = (D + 1) / 2;
+  constexpr int E = kBasis<D>, D2 = (E + 1) / 2;
   __shared__ GeoSlot geo[2 * kPairThreads];
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   const int a = gt / TPA;
@@ -99,15 +89,13 @@ k_force(KParams kp, BoxP box, int n, int cap, float scale,
       for (int q = 0; q < 4; q++) {
         float gp[4];
         dedp_row_g(G, dEdG, row0 + q, kp.M, gp);
-        const float *Pp = P + (row0 + q) * D;
+        float A[E], F[2 * D2];
 #pragma unroll
-        for (int p = 0; p < D2; p++) {
-          const float s0 = dedp_elem(gp, kp.T, D, kp.M, 2 * p, __ldg(Pp + 2 * p));
-          const float s1 = 2 * p + 1 < D
-                               ? dedp_elem(gp, kp.T, D, kp.M, 2 * p + 1, __ldg(Pp + 2 * p + 1))
-                               : 0.f;
-          S2[q][p] = make_float2(s0, s1);
-        }
+        for (int d = 0; d < E; d++) A[d] = __ldg(P + (row0 + q) * E + d);
+        dedp_row<D>(gp, kp.T, kp.M, A, F);
+        if (E & 1) F[E] = 0.f;
+#pragma unroll
+        for (int p = 0; p < D2; p++) S2[q][p] = make_float2(F[2 * p], F[2 * p + 1]);
       }
     }
     float4 *pdf_row = pdf + (size_t)a * cap;
@@ -122,7 +110,7 @@ k_force(KParams kp, BoxP box, int n, int cap, float scale,
         float H[4], dH[4];
         radial4<RK, true>(kp, R, g, H, dH);
         float2 M2[D2];
-        moments2<D, D2>(g.ux, g.uy, g.uz, M2);
+        moments2<D, D2, true>(g.ux, g.uy, g.uz, M2);
         // V_d = sum_k S[k,d] H_k and W_d = sum_k S[k,d] dH_k: 2 x D2
         // independent FFMA2 chains of length 4; then the F1 scalar
         // sum_k U_k dH_k = sum_d M_d W_d as two interleaved partial dots

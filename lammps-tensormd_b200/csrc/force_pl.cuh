@@ -2,7 +2,7 @@
 //
 // Same mathematics and outputs as k_force (force_impl.cuh): S = dE/dP of each
 // (atom, element block) formed from P, G and dE/dG when the group reaches the
-// block (dedp_row_g / dedp_elem), then for every active
+// block (dedp_row_g / dedp_row), then for every active
 // pair of atom i, V_d = sum_k S[k,d] H_k, W_d = sum_k S[k,d] dH_k,
 // df = (sum_d M_d W_d) u + grad Q(V) / r, scaled, into pdf[i*cap + t]; FP64
 // per-atom virial into wv[i].
@@ -11,7 +11,7 @@
 // forces, so every lane of the atom's group evaluates the monomials, the
 // gradient of Q and the force expression of every pair.  Here W lanes share
 // one atom and each lane takes whole pairs: S of the current element block
-// (K x D floats) is staged once in shared memory and read by all lanes of the
+// (K x E floats, E = kBasis<D>) is staged once in shared memory and read by all lanes of the
 // group as broadcast vectors, and the monomials, grad Q and the force of a
 // pair are computed once.  The pairs are the compact list of active pairs
 // that the descriptor step wrote (pgeo, pcnt: geometry computed once per
@@ -27,16 +27,15 @@
 namespace tmd {
 
 // Shared-memory layout of k_force_pl (floats): radial parameters [4][K] (none
-// for the table kind) and T [4][D4], then per atom group an S block [K][D4]
-// + 4 (the extra 4 floats put consecutive groups' blocks in different banks)
-// and the dE/dG' rows [K][4].
+// for the table kind), then per atom group an S block [K][D4] + 4 (the extra 4
+// floats put consecutive groups' blocks in different banks).
 template <int D>
 struct PlLayout {
-  static constexpr int D4 = (D + 3) / 4 * 4;
+  static constexpr int D4 = (kBasis<D> + 3) / 4 * 4;
   static __host__ __device__ inline int params(int K, int rk) {
-    return (rk == kRadTable ? 0 : 4 * K) + 4 * D4;
+    return rk == kRadTable ? 0 : 4 * K;
   }
-  static __host__ __device__ inline int group(int K) { return K * D4 + 4 + 4 * K; }
+  static __host__ __device__ inline int group(int K) { return K * D4 + 4; }
   static __host__ inline size_t bytes(int K, int rk, int groups) {
     return sizeof(float) * ((size_t)params(K, rk) + (size_t)groups * group(K));
   }
@@ -56,16 +55,11 @@ k_force_pl(KParams kp, BoxP box, int n, int cap, float scale,
            const int *__restrict__ acell, const float4 *__restrict__ pgeo,
            const int *__restrict__ pcnt) {
   using L = PlLayout<D>;
-  constexpr int D4 = L::D4;
+  constexpr int D4 = L::D4, E = kBasis<D>;
   constexpr int P2 = D4 / 2;  // FP32 pairs per S row (pad columns hold 0)
   extern __shared__ float4 pl_dyn[];
   const int K = KC > 0 ? KC : kp.K, B = kp.B, M = kp.M;
   float *rp = reinterpret_cast<float *>(pl_dyn);
-  float *Ts = rp + (RK == kRadTable ? 0 : 4 * K);  // T[m][d], rows of D4
-  for (int i = threadIdx.x; i < 4 * D4; i += blockDim.x) {
-    const int m = i / D4, d = i - m * D4;
-    Ts[i] = (m < M && d < D) ? kp.T[m * D + d] : 0.f;
-  }
   if (RK != kRadTable) {
     for (int i = threadIdx.x; i < K; i += blockDim.x) {
       rp[i] = RK == kRadGauss ? kp.p1[i] : kp.p0[i];
@@ -83,7 +77,6 @@ k_force_pl(KParams kp, BoxP box, int n, int cap, float scale,
   const int lane = threadIdx.x & 31;
   const unsigned gmask = PairRing<W>::kBits << (lane & ~(W - 1));
   float *Sg = rp + L::params(K, RK) + (threadIdx.x / W) * L::group(K);
-  float *gpg = Sg + K * D4 + 4;  // dE/dG' rows [K][4]
   const float4 *pg_row = pgeo + (size_t)a * cap * 2;
   float4 *pdf_row = pdf + (size_t)a * cap;
   float w6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -92,52 +85,45 @@ k_force_pl(KParams kp, BoxP box, int n, int cap, float scale,
     if (b > 0) __syncwarp(live);  // keep the warp's groups on the same block
     const int np = pcnt[(size_t)a * B + b];
     if (np == 0) continue;
-    // S = dE/dP of (atom, block) as [K][D4] rows: dE/dG' rows first, then
-    // one element per lane step (same arithmetic and order as dedp_elem)
-    __syncwarp(gmask);
-    const size_t row0 = ((size_t)a * B + b) * K;
-    for (int k = sub; k < K; k += W) {
-      float gp[4];
-      dedp_row_g(G, dEdG, row0 + k, M, gp);
-      *reinterpret_cast<float4 *>(gpg + 4 * k) = make_float4(gp[0], gp[1], gp[2], gp[3]);
-    }
+    // S = dE/dP of (atom, block), folded to Q's coefficients, as [K][D4]
+    // rows: one filter per lane, the loads of kRows filters in flight
     __syncwarp(gmask);
     {
-      // 4-column units of the [K][D4] block, kBatch P loads in flight per lane
-      constexpr int kBatch = 4;
-      const int nv = K * D4 / 4;
-      for (int v0 = sub; v0 < nv; v0 += W * kBatch) {
-        float4 pv[kBatch];
+      constexpr int kRows = 2;
+      const size_t row0 = ((size_t)a * B + b) * K;
+      for (int k0 = sub; k0 < K; k0 += W * kRows) {
+        float gp[kRows][4], A[kRows][E];
 #pragma unroll
-        for (int u = 0; u < kBatch; u++) {
-          const int v = v0 + u * W;
-          pv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (v < nv) {
-            const int k = (4 * v) / D4, d0 = 4 * v - k * D4;
-            const float *Pr = P + (row0 + k) * D;
-            if constexpr (D == D4) {
-              pv[u] = __ldg(reinterpret_cast<const float4 *>(Pr + d0));
+        for (int u = 0; u < kRows; u++) {
+          const int k = k0 + u * W;
+          if (k < K) {
+            const float *Pr = P + (row0 + k) * E;
+            if constexpr (E % 4 == 0) {
+#pragma unroll
+              for (int v = 0; v < E / 4; v++) {
+                const float4 p = __ldg(reinterpret_cast<const float4 *>(Pr) + v);
+                A[u][4 * v] = p.x; A[u][4 * v + 1] = p.y;
+                A[u][4 * v + 2] = p.z; A[u][4 * v + 3] = p.w;
+              }
             } else {
-              pv[u].x = d0 < D ? __ldg(Pr + d0) : 0.f;
-              pv[u].y = d0 + 1 < D ? __ldg(Pr + d0 + 1) : 0.f;
-              pv[u].z = d0 + 2 < D ? __ldg(Pr + d0 + 2) : 0.f;
-              pv[u].w = d0 + 3 < D ? __ldg(Pr + d0 + 3) : 0.f;
+#pragma unroll
+              for (int d = 0; d < E; d++) A[u][d] = __ldg(Pr + d);
             }
+            dedp_row_g(G, dEdG, row0 + k, M, gp[u]);
           }
         }
 #pragma unroll
-        for (int u = 0; u < kBatch; u++) {
-          const int v = v0 + u * W;
-          if (v < nv) {
-            const int k = (4 * v) / D4, d0 = 4 * v - k * D4;
-            const float4 g4 = *reinterpret_cast<const float4 *>(gpg + 4 * k);
-            const float gp[4] = {g4.x, g4.y, g4.z, g4.w};
-            const float p[4] = {pv[u].x, pv[u].y, pv[u].z, pv[u].w};
-            float s[4];
+        for (int u = 0; u < kRows; u++) {
+          const int k = k0 + u * W;
+          if (k < K) {
+            float F[D4];
+            dedp_row<D>(gp[u], kp.T, M, A[u], F);
 #pragma unroll
-            for (int j = 0; j < 4; j++)
-              s[j] = d0 + j < D ? dedp_elem(gp, Ts, D4, M, d0 + j, p[j]) : 0.f;
-            *reinterpret_cast<float4 *>(Sg + 4 * v) = make_float4(s[0], s[1], s[2], s[3]);
+            for (int d = E; d < D4; d++) F[d] = 0.f;
+#pragma unroll
+            for (int v = 0; v < D4 / 4; v++)
+              *reinterpret_cast<float4 *>(Sg + k * D4 + 4 * v) =
+                  make_float4(F[4 * v], F[4 * v + 1], F[4 * v + 2], F[4 * v + 3]);
           }
         }
       }
@@ -206,9 +192,9 @@ k_force_pl(KParams kp, BoxP box, int n, int cap, float scale,
           }
         }
         float M[D4];
-        moments<D>(g.ux, g.uy, g.uz, M);
+        basis_q<D>(g.ux, g.uy, g.uz, M);
 #pragma unroll
-        for (int d = D; d < D4; d++) M[d] = 0.f;
+        for (int d = E; d < D4; d++) M[d] = 0.f;
         float2 fa = make_float2(0.f, 0.f), fb = make_float2(0.f, 0.f);
 #pragma unroll
         for (int p = 0; p < P2; p += 2) {

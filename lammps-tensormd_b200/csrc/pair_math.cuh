@@ -306,42 +306,170 @@ __device__ inline void moments(float x, float y, float z, float M[D]) {
   }
 }
 
-// Gradient of Q(u) = sum_d V_d M_d(u) with respect to u, and sum_d n_d V_d M_d
-// (n_d = rank of monomial d).  Then dQ/dx_j = (gradQ - u * nVM) / r, which
-// is sum_d V_d dM_d/dx_j (tensor_ops.cpp calculate_dM_{p,d,f}).  Each M_d is
-// homogeneous of degree n_d, so u . grad M_d = n_d M_d (Euler) and nVM is
-// formed as u . gradQ.
+// Rank 3: 16 functions in place of 20 monomials.  u is a unit vector, so
+// xx + yy + zz = 1 and the 20 monomials span only 16 functions on the sphere:
+// four of every five FMAs of the contractions and of the shared-memory reads
+// that feed them, and rows of 64 bytes.  The descriptor accumulates P over the
+// orthogonal set {1, x, y, z, zz - 1/3, xy, xz, xx - yy, yz, x (xx - 3/5),
+// x (yy - zz), y (yy - 3/5), y (zz - xx), z (zz - 3/5), z (xx - yy), xyz}: a
+// monomial's sum, put together again from orthogonal parts, carries the
+// rounding noise of its direct sum and no more (with xx - zz and the like,
+// sums over xyy came out 1.5 times as noisy).  The pair force evaluates Q(u)
+// with zz eliminated, over {1, x, y, z, xx, xy, xz, yy, yz, xxx, xxy, xxz,
+// xyy, xyz, yyy, yyz}.
 template <int D>
-__device__ inline void poly_grad(const float V[D], float x, float y, float z,
+constexpr int kBasis = basis_count(D);
+
+template <int D>
+__device__ inline void basis_p(float x, float y, float z, float M[kBasis<D>]) {
+  if constexpr (D < 20) {
+    moments<D>(x, y, z, M);
+  } else {
+    const float xx = x * x, yy = y * y, zz = z * z, xy = x * y;
+    M[0] = 1.f; M[1] = x; M[2] = y; M[3] = z;
+    M[4] = fmaf(z, z, -1.f / 3.f); M[5] = xy; M[6] = x * z; M[7] = (x - y) * (x + y); M[8] = y * z;
+    M[9] = x * (xx - 0.6f); M[10] = x * (yy - zz); M[11] = y * (yy - 0.6f);
+    M[12] = y * (zz - xx); M[13] = z * (zz - 0.6f); M[14] = z * (xx - yy); M[15] = xy * z;
+  }
+}
+
+// The sums over monomials that the 16 sums stand for.
+struct Rank3 {
+  float xx, yy, zz, xxx, xyy, xzz, xxy, yyy, yzz, xxz, yyz, zzz;
+};
+__device__ inline Rank3 basis_expand(const float A[16]) {
+  Rank3 r;
+  const float t = A[0] * (1.f / 3.f);
+  r.zz = t + A[4];
+  r.xx = fmaf(0.5f, A[7] - A[4], t);
+  r.yy = fmaf(-0.5f, A[7] + A[4], t);
+  r.xxx = fmaf(0.6f, A[1], A[9]);
+  r.xyy = fmaf(0.2f, A[1], 0.5f * (A[10] - A[9]));
+  r.xzz = fmaf(0.2f, A[1], -0.5f * (A[10] + A[9]));
+  r.yyy = fmaf(0.6f, A[2], A[11]);
+  r.yzz = fmaf(0.2f, A[2], 0.5f * (A[12] - A[11]));
+  r.xxy = fmaf(0.2f, A[2], -0.5f * (A[12] + A[11]));
+  r.zzz = fmaf(0.6f, A[3], A[13]);
+  r.xxz = fmaf(0.2f, A[3], 0.5f * (A[14] - A[13]));
+  r.yyz = fmaf(0.2f, A[3], -0.5f * (A[14] + A[13]));
+  return r;
+}
+
+// G row of one (atom, block, filter): G_m = sum_d T[m][d] P_d^2, G_0 with the
+// sign of P_0 under a square root (kernel_1_fused_device, kernel.cu:1028-1061).
+// T depends on a monomial only through its exponents' partition (1; x; xx, xy;
+// xxx, xxy, xyz), so rank 3 sums the squares of each class first.
+template <int D, int M>
+__device__ inline void invariants(const float A[kBasis<D>], const float *T, float G[M]) {
+  if constexpr (D < 20) {
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      float s = 0.f;
+#pragma unroll
+      for (int d = 0; d < D; d++) s = fmaf(T[m * D + d], A[d] * A[d], s);
+      G[m] = s;
+    }
+  } else {
+    const Rank3 p = basis_expand(A);
+    const float c0 = A[0] * A[0];
+    const float c1 = fmaf(A[3], A[3], fmaf(A[2], A[2], A[1] * A[1]));
+    const float c4 = fmaf(p.zz, p.zz, fmaf(p.yy, p.yy, p.xx * p.xx));
+    const float c5 = fmaf(A[8], A[8], fmaf(A[6], A[6], A[5] * A[5]));
+    const float c10 = fmaf(p.zzz, p.zzz, fmaf(p.yyy, p.yyy, p.xxx * p.xxx));
+    const float c11 = fmaf(p.xzz, p.xzz, fmaf(p.yzz, p.yzz, fmaf(p.xyy, p.xyy, fmaf(p.xxy, p.xxy,
+                      fmaf(p.xxz, p.xxz, p.yyz * p.yyz)))));
+    const float c14 = A[15] * A[15];
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      const float *t = T + m * D;
+      G[m] = fmaf(t[0], c0, fmaf(t[1], c1, fmaf(t[4], c4, fmaf(t[5], c5, fmaf(t[10], c10,
+             fmaf(t[11], c11, t[14] * c14))))));
+    }
+  }
+  G[0] = copysignf(1.f, A[0]) * sqrtf(G[0]);
+}
+
+// Coefficients of Q(u) for one filter: S_d = dE/dP_d = 2 P_d sum_m T[m][d]
+// gp_m (kernel2_GPU, kernel.cu:730-848), for rank 3 folded to the 16
+// functions that the force evaluates (zz = 1 - xx - yy).
+template <int D>
+__device__ inline void dedp_row(const float gp[4], const float *T, int M,
+                                const float A[kBasis<D>], float F[kBasis<D>]) {
+  auto t2 = [&](int d) {
+    float t = 0.f;
+#pragma unroll
+    for (int m = 0; m < 4; m++)
+      if (m < M) t = fmaf(gp[m], T[m * D + d], t);
+    return 2.f * t;
+  };
+  if constexpr (D < 20) {
+#pragma unroll
+    for (int d = 0; d < D; d++) F[d] = t2(d) * A[d];
+  } else {
+    const Rank3 p = basis_expand(A);
+    const float t0 = t2(0), t1 = t2(1), t4 = t2(4), t5 = t2(5), t10 = t2(10), t11 = t2(11),
+                t14 = t2(14);
+    F[0] = fmaf(t4, p.zz, t0 * A[0]);
+    F[1] = fmaf(t11, p.xzz, t1 * A[1]);
+    F[2] = fmaf(t11, p.yzz, t1 * A[2]);
+    F[3] = fmaf(t10, p.zzz, t1 * A[3]);
+    F[4] = t4 * fmaf(-1.5f, A[4], 0.5f * A[7]);
+    F[5] = t5 * A[5];
+    F[6] = t5 * A[6];
+    F[7] = t4 * fmaf(-1.5f, A[4], -0.5f * A[7]);
+    F[8] = t5 * A[8];
+    F[9] = fmaf(t10, p.xxx, -t11 * p.xzz);
+    F[10] = -t11 * A[12];
+    F[11] = fmaf(t11, p.xxz, -t10 * p.zzz);
+    F[12] = t11 * A[10];
+    F[13] = t14 * A[15];
+    F[14] = fmaf(t10, p.yyy, -t11 * p.yzz);
+    F[15] = fmaf(t11, p.yyz, -t10 * p.zzz);
+  }
+}
+
+// The functions of Q(u).
+template <int D>
+__device__ inline void basis_q(float x, float y, float z, float M[kBasis<D>]) {
+  if constexpr (D < 20) {
+    moments<D>(x, y, z, M);
+  } else {
+    const float xx = x * x, xy = x * y, xz = x * z, yy = y * y, yz = y * z;
+    M[0] = 1.f; M[1] = x; M[2] = y; M[3] = z;
+    M[4] = xx; M[5] = xy; M[6] = xz; M[7] = yy; M[8] = yz;
+    M[9] = xx * x; M[10] = xx * y; M[11] = xx * z; M[12] = yy * x; M[13] = xy * z;
+    M[14] = yy * y; M[15] = yy * z;
+  }
+}
+
+// Gradient of Q(u) = sum_d V_d M_d(u) with respect to u, and u . grad Q.  Then
+// dQ/dx_j = (gradQ - u (u . gradQ)) / r, which is sum_d V_d dM_d/dx_j
+// (tensor_ops.cpp calculate_dM_{p,d,f}): only the tangential part counts, so
+// Q may be any polynomial with the right values on the sphere.
+template <int D>
+__device__ inline void poly_grad(const float V[kBasis<D>], float x, float y, float z,
                                  float gq[3], float &nvm) {
   // Horner form: grad_a Q = V_a + x P_a + y Q_a + z R_a, with P, Q, R the
   // coefficients of x, y, z once the linear terms are taken out (three short
   // independent chains instead of one long sum per component)
   float gx = 0.f, gy = 0.f, gz = 0.f;
-  if (D > 1) {
-    float Px = 0.f, Qx = 0.f, Rx = 0.f, Py = 0.f, Qy = 0.f, Ry = 0.f, Pz = 0.f, Qz = 0.f,
-          Rz = 0.f;
-    if (D > 4) {
-      // xx, xy, xz, yy, yz, zz
-      Px = 2.f * V[4]; Qx = V[5]; Rx = V[6];
-      Py = V[5]; Qy = 2.f * V[7]; Ry = V[8];
-      Pz = V[6]; Qz = V[8]; Rz = 2.f * V[9];
-      if (D > 10) {
-        // xxx xxy xxz xyy xyz xzz yyy yyz yzz zzz
-        Px = fmaf(3.f * V[10], x, fmaf(2.f * V[11], y, fmaf(2.f * V[12], z, Px)));
-        Qx = fmaf(V[13], y, fmaf(V[14], z, Qx));
-        Rx = fmaf(V[15], z, Rx);
-        Py = fmaf(V[11], x, fmaf(2.f * V[13], y, fmaf(V[14], z, Py)));
-        Qy = fmaf(3.f * V[16], y, fmaf(2.f * V[17], z, Qy));
-        Ry = fmaf(V[18], z, Ry);
-        Pz = fmaf(V[12], x, fmaf(V[14], y, fmaf(2.f * V[15], z, Pz)));
-        Qz = fmaf(V[17], y, fmaf(2.f * V[18], z, Qz));
-        Rz = fmaf(3.f * V[19], z, Rz);
-      }
-    }
-    gx = fmaf(x, Px, fmaf(y, Qx, fmaf(z, Rx, V[1])));
-    gy = fmaf(x, Py, fmaf(y, Qy, fmaf(z, Ry, V[2])));
-    gz = fmaf(x, Pz, fmaf(y, Qz, fmaf(z, Rz, V[3])));
+  if constexpr (D == 4) {
+    gx = V[1]; gy = V[2]; gz = V[3];
+  } else if constexpr (D == 10) {
+    // xx, xy, xz, yy, yz, zz
+    gx = fmaf(x, 2.f * V[4], fmaf(y, V[5], fmaf(z, V[6], V[1])));
+    gy = fmaf(x, V[5], fmaf(y, 2.f * V[7], fmaf(z, V[8], V[2])));
+    gz = fmaf(x, V[6], fmaf(y, V[8], fmaf(z, 2.f * V[9], V[3])));
+  } else if constexpr (D == 20) {
+    const float Px = fmaf(3.f * V[9], x, fmaf(2.f * V[10], y, fmaf(2.f * V[11], z, 2.f * V[4])));
+    const float Qx = fmaf(V[12], y, fmaf(V[13], z, V[5]));
+    const float Py = fmaf(V[10], x, fmaf(2.f * V[12], y, fmaf(V[13], z, V[5])));
+    const float Qy = fmaf(3.f * V[14], y, fmaf(2.f * V[15], z, 2.f * V[7]));
+    const float Pz = fmaf(V[11], x, fmaf(V[13], y, V[6]));
+    const float Qz = fmaf(V[15], y, V[8]);
+    gx = fmaf(x, Px, fmaf(y, Qx, fmaf(z, V[6], V[1])));
+    gy = fmaf(x, Py, fmaf(y, Qy, fmaf(z, V[8], V[2])));
+    gz = fmaf(x, Pz, fmaf(y, Qz, V[3]));
   }
   gq[0] = gx; gq[1] = gy; gq[2] = gz;
   nvm = x * gx + y * gy + z * gz;

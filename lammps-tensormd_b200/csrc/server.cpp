@@ -129,7 +129,7 @@ size_t server_bytes_per_atom(const tmd_model *m, int cap) {
   size_t a = 4 * 24 + 12 + 4;          // x, v, f, xbuild; image; element
   a += 3 * 4;                          // bin of atom, binned atoms, raw row length
   a += 4 * (B + 1) + 4 * B;            // row block offsets, active pairs per block
-  a += 4 * B * h.K * h.D + 2 * 4 * nin;  // P; G and dE/dG
+  a += 4 * B * h.K * basis_count(h.D) + 2 * 4 * nin;  // P; G and dE/dG
   a += 8 + 48 + 8 + 48 + 8 + 4 + 4;    // E, virial partials, eatom, vatom, ke, perm, cell
   a += 4 * 24 + 12 + 4 + 4 * (B + 1);  // relayout copies: x v f xbuild, image, element, offsets
   a += 48 + 4 + 40 + 8;                // staging x v, staging element, FIRE power and maxima, |F|^2

@@ -10,6 +10,9 @@ constexpr int kMaxElt = 8;      // potential elements (reference MAX_ELETYPES 5)
 constexpr int kMaxK = 128;      // radial filters
 constexpr int kMaxD = 20;       // monomials of rank <= 3
 constexpr int kMaxLayers = 12;  // MLP layers
+// functions that P is kept over: the D monomials, for rank 3 the 16 that are
+// independent on the unit sphere (pair_math.cuh)
+constexpr int basis_count(int D) { return D == 20 ? 16 : D; }
 constexpr int kShiftR = 3;      // periodic image shift range [-3, 3] per axis
 constexpr int kShiftBits = 9;   // 7^3 = 343 codes
 constexpr int kAtomBits = 23;   // atom index bits of a neighbor entry
