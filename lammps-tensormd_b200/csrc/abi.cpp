@@ -351,11 +351,15 @@ DescArgs desc_args(tmd_system *s, int variant) {
   return d;
 }
 
-int default_desc_variant(const tmd_model *m) {
-  // measured on the B200 (tmd_system_autotune): the wide form is 1.25-1.33x
-  // faster at K = 16 and equal at K = 32
-  (void)m;
-  return kDescWide;
+// The descriptor form in use: the caller's or the autotuner's choice, else the
+// wide form, and for table radials on many atoms the split one (measured on
+// the B200, k_pair_geo + k_descriptor_c against k_descriptor_w: 23,040 atoms
+// of a 32-filter table potential 162 against 187 us; at 430 atoms the second
+// launch costs more than it gives, and the Gaussian kinds gain under 3%).
+// Both sum the pairs in the same order: the results are the same bit for bit.
+int desc_form(const tmd_system *s) {
+  if (s->desc_variant >= 0) return s->desc_variant;
+  return s->m->kp.radial == 1 && s->n >= 8192 ? kDescSplit : kDescWide;
 }
 
 int default_force_variant(const tmd_model *m) {
@@ -379,7 +383,7 @@ ForceArgs force_args(tmd_system *s, float scale, int variant) {
 
 void launch_force_eval(tmd_system *s, float scale, bool want_vatom) {
   const tmd_model *m = s->m;
-  const DescArgs d = desc_args(s, s->desc_variant);
+  const DescArgs d = desc_args(s, desc_form(s));
   prof_begin(s);
   launch_descriptor(d, s->st, s->launches);
   prof_end(s, 1);
@@ -1230,7 +1234,6 @@ int tmd_system_create(const tmd_model *m, int natoms_cap, double skin,
   s->natoms_cap = natoms_cap;
   s->skin = skin;
   s->force_variant = default_force_variant(m);
-  s->desc_variant = default_desc_variant(m);
   s->etemp = m->h.etemp;
   const HostModel &h = m->h;
   size_t N = natoms_cap;
@@ -1620,7 +1623,7 @@ int tmd_get_descriptors(tmd_system *s, double *G) {
   // the descriptor of the current positions (compute tensormd/density runs
   // between force evaluations, after LAMMPS moved the atoms)
   for (int attempt = 0; attempt < 2; attempt++) {
-    launch_descriptor(desc_args(s, s->desc_variant), s->st, s->launches);
+    launch_descriptor(desc_args(s, desc_form(s)), s->st, s->launches);
     TMD_CUDA(cudaGetLastError());
     int rc = read_status(s);
     if (rc) return rc;
@@ -1661,7 +1664,7 @@ int tmd_system_set_variant(tmd_system *s, int family, int variant) {
 int tmd_system_get_variant(tmd_system *s, int family, int *variant) {
   if (!s || !variant) return fail(TMD_ERR_ARG, "null argument");
   if (family_forms(family) == 0) return fail(TMD_ERR_ARG, "unknown kernel family");
-  *variant = family_slot(s, family);
+  *variant = family == TMD_TUNE_DESCRIPTOR ? desc_form(s) : s->force_variant;
   return TMD_OK;
 }
 

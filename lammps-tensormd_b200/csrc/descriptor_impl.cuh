@@ -26,6 +26,10 @@
 namespace tmd {
 
 constexpr int kPairThreads = 128;  // block size of the pair kernels
+// Pairs in flight of the descriptor's contraction loops: the table kinds wait
+// for each pair's table row (an L2 access), so they take four at a time.
+template <int RK>
+constexpr int kPairUnroll = RK == kRadTable ? 4 : 2;
 
 // Geometry slot in shared memory: three 16-byte vectors per lane; the inputs
 // of the radial basis (r, r_lo, f_c, table offset) share the first, so the
@@ -193,7 +197,7 @@ __device__ inline PairGeo decode_pair_geo(const float4 a, const float4 b, int &t
     g.fc = b.y; g.dfc = b.z; g.ti = 0; g.tq = 0.f;
   }
   t = __float_as_int(b.w);
-  g.rinv = __frcp_rn(g.r);  // 1/r rounded to nearest, as pair_geometry
+  g.rinv = rcp_newton(g.r);
   return g;
 }
 
@@ -203,8 +207,9 @@ __device__ inline PairGeo load_pair_geo(const float4 *__restrict__ src, int &t) 
 }
 
 // P_0 = sum_j H_k, by far the largest of a filter's sums and the one whose
-// rounding reaches G_0 and G_2 together, is summed chunk by chunk: the chunk's
-// sum starts from zero and is folded into p0 at the end of the chunk.  On BCC
+// rounding reaches G_0 and G_2 together, is summed in runs of 16 pairs: a run
+// starts from zero and is folded into p0 at its end (the same runs in every
+// one-stream form, so their sums agree bit for bit).  On BCC
 // cells this takes the descriptor's share of the force error from 2.8e-6 (one
 // running sum, 20 monomials) to 1.7e-6.
 template <int F, int N>
@@ -218,7 +223,7 @@ __device__ __forceinline__ void fold_p0(float2 (&acc)[F][N], float (&p0)[F]) {
 template <int F, int N>
 __device__ __forceinline__ void take_p0(float2 (&acc)[F][N], const float (&p0)[F]) {
 #pragma unroll
-  for (int f = 0; f < F; f++) acc[f][0].x = p0[f];
+  for (int f = 0; f < F; f++) acc[f][0].x += p0[f];
 }
 
 template <int TPA, int D, int RK, bool MULTI>
@@ -284,7 +289,7 @@ k_descriptor(KParams kp, BoxP box, int n, int cap, const double *__restrict__ x,
         }
       }
       pr.pop(cnt);
-      fold_p0(acc, p0);
+      if (((nact - nact0) & 15) == 0) fold_p0(acc, p0);
     }
     take_p0(acc, p0);
     if (sub == 0) pcnt[(size_t)a * B + b] = nact - nact0;
@@ -379,8 +384,11 @@ k_descriptor_w(KParams kp, BoxP box, int n, int cap, const double *__restrict__ 
       if (cnt == 0) break;
       if (sub < cnt) store_pair_geo<RK>(pr.slot(sub), pg_row + 2 * (nact + sub));
       nact += cnt;
-#pragma unroll 2
-      for (int c = 0; c < cnt; c++) {
+      constexpr int kRun = W < 16 ? W : 16;
+      for (int h = 0; h < cnt; h += kRun) {
+      const int ce = min(cnt, h + kRun);
+#pragma unroll kPairUnroll<RK>
+      for (int c = h; c < ce; c++) {
         const PairGeo g = geo_load_radial<RK>(pr.slot(c));
         const float4 *ms = reinterpret_cast<const float4 *>(
             mr + ((pr.head + c) & (PairRing<W>::kSlots - 1)) * D4);
@@ -401,8 +409,9 @@ k_descriptor_w(KParams kp, BoxP box, int n, int cap, const double *__restrict__ 
           }
         }
       }
+      if (((nact - cnt - nact0 + ce) & 15) == 0) fold_p0(acc, p0);
+      }
       pr.pop(cnt);
-      fold_p0(acc, p0);
     }
     take_p0(acc, p0);
     if (sub == 0) pcnt[(size_t)a * B + b] = nact - nact0;
@@ -597,7 +606,7 @@ void launch_descriptor_w2(const DescArgs &a, cudaStream_t st) {
 // Warp per atom: entries of each element block in rounds of 32, active ones
 // compacted in row order (ballot + prefix count).
 template <int RK, bool MULTI>
-__global__ void __launch_bounds__(256, 6)
+__global__ void __launch_bounds__(256, 5)
 k_pair_geo(KParams kp, BoxP box, int n, int cap, const double *__restrict__ x,
            const uint32_t *__restrict__ nbr, const int *__restrict__ boff,
            const BoxP *__restrict__ cbox, const int *__restrict__ acell,
@@ -655,7 +664,7 @@ k_pair_geo(KParams kp, BoxP box, int n, int cap, const double *__restrict__ x,
 // buffers, so one warp sync per chunk); every lane then accumulates its
 // filters over the chunk's pairs in row order, as k_descriptor_w.
 template <int W, int FPL, int D, int RK>
-__global__ void __launch_bounds__(kPairThreads, 8)
+__global__ void __launch_bounds__(kPairThreads, FPL == 1 ? 8 : 6)
 k_descriptor_c(KParams kp, int n, int cap, float *__restrict__ P, float *__restrict__ G,
                const float4 *__restrict__ pgeo, const int *__restrict__ pcnt) {
   constexpr int E = kBasis<D>, D4 = (E + 3) / 4 * 4;
@@ -718,8 +727,11 @@ k_descriptor_c(KParams kp, int n, int cap, float *__restrict__ P, float *__restr
       }
       __syncwarp(gmask);
       const float *cs = sg + buf * W * SL;
-#pragma unroll 2
-      for (int c = 0; c < cnt; c++) {
+      constexpr int kRun = W < 16 ? W : 16;
+      for (int h = 0; h < cnt; h += kRun) {
+      const int ce = min(cnt, h + kRun);
+#pragma unroll kPairUnroll<RK>
+      for (int c = h; c < ce; c++) {
         const float4 *ms = reinterpret_cast<const float4 *>(cs + c * SL);
         const float4 rr = ms[D4 / 4];
         PairGeo g;
@@ -748,8 +760,9 @@ k_descriptor_c(KParams kp, int n, int cap, float *__restrict__ P, float *__restr
           }
         }
       }
+      if (((c0 + ce) & 15) == 0) fold_p0(acc, p0);
+      }
       buf ^= 1;
-      fold_p0(acc, p0);
     }
     take_p0(acc, p0);
     pos += np;
@@ -868,9 +881,9 @@ void launch_descriptor_rk(const DescArgs &a, cudaStream_t st) {
   if (a.variant == kDescSplit) {
     switch (a.kp.K) {
       case 4: launch_descriptor_split<4, 1, RK, MULTI>(a, st); break;
-      case 8: launch_descriptor_split<8, 1, RK, MULTI>(a, st); break;
-      case 16: launch_descriptor_split<16, 1, RK, MULTI>(a, st); break;
-      case 32: launch_descriptor_split<32, 1, RK, MULTI>(a, st); break;
+      case 8: launch_descriptor_split<4, 2, RK, MULTI>(a, st); break;
+      case 16: launch_descriptor_split<8, 2, RK, MULTI>(a, st); break;
+      case 32: launch_descriptor_split<16, 2, RK, MULTI>(a, st); break;
       case 64: launch_descriptor_split<32, 2, RK, MULTI>(a, st); break;
       default: launch_descriptor_split<32, 4, RK, MULTI>(a, st); break;
     }

@@ -152,6 +152,10 @@ k_force_pl(KParams kp, BoxP box, int n, int cap, float scale,
           W2[p] = make_float2(0.f, 0.f);
         }
         const bool on = RK != kRadTable || (g.ti > 0 && g.ti < kp.tab_n - 2);
+        // table kinds: the row of the next four filters is fetched while the
+        // current ones are contracted
+        TabRow tab{};
+        if (RK == kRadTable && on) tab = load_tab(kp, g.ti, 0);
 #pragma unroll
         for (int k0 = 0; k0 < (KC > 0 ? KC : K); k0 += 4) {
           if (!on) break;
@@ -174,7 +178,13 @@ k_force_pl(KParams kp, BoxP box, int n, int cap, float scale,
             }
           }
           float H[4], dH[4];
-          radial4<RK, true>(kp, R, g, H, dH);
+          if constexpr (RK == kRadTable) {
+            const TabRow cur = tab;
+            if (k0 + 4 < (KC > 0 ? KC : K)) tab = load_tab(kp, g.ti, k0 + 4);
+            tab_eval4(kp, cur, g.tq, true, H, dH);
+          } else {
+            radial4<RK, true>(kp, R, g, H, dH);
+          }
 #pragma unroll
           for (int q = 0; q < 4; q++) {
             const float2 h2 = make_float2(H[q], H[q]);

@@ -28,7 +28,7 @@
 //
 // Measured on the B200 against the kernels it replaced (a warp-tile form, a
 // resident-weight form and a streamed form with 64- to 512-atom tiles), same
-// sums bit for bit: 16 atoms of a 512-64x4 residual net 111 -> 40 us, 4,000
+// sums bit for bit and before the activations below: 16 atoms of a 512-64x4 residual net 111 -> 40 us, 4,000
 // atoms 64-64-64 49 -> 14, 23,040 atoms 128-128x3 residual 270 -> 169, 128,000
 // atoms 64-64-64 180 -> 160, 432,000 atoms 512-128x3 5.86 -> 4.50 ms (56% of
 // the FP32 peak).  The producer needs a warp of its own: in a consumer warp
@@ -52,34 +52,82 @@ constexpr int kMlpThreads = 128;  // consumers: the threads of the GEMMs and epi
 constexpr int kMlpBlock = kMlpThreads + 32;  // and one producer warp
 constexpr int kMlpPad = 32;  // reduction rows of the packed weights are padded to this
 
-__device__ inline float mlp_act(int actfn, float z, float &d) {
+// 1/u and a/u, to about half an ulp, for u between 1 and 2^60: the
+// approximate reciprocal and one Newton step, without the scaling that the
+// full-range division needs.
+__device__ __forceinline__ float mlp_rcp(float u) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(u));
+  return fmaf(r, fmaf(-u, r, 1.f), r);
+}
+__device__ __forceinline__ float mlp_div(float a, float u, float rcp_u) {
+  const float q = a * rcp_u;
+  return fmaf(fmaf(-q, u, a), rcp_u, q);
+}
+
+// Activation and its derivative (nnp.cu:9-57), each from one exponential (or
+// square root) and one or two reciprocals, branch-free: the epilogues were a
+// sixth to a third of the kernel with expf, tanhf or log1pf and IEEE divisions
+// (432,000-atom alloy, softplus: 4.50 -> 3.91 ms; 23,040-atom W net,
+// squareplus: 169 -> 143 us; 128,000 atoms, tanh: 160 -> 145 us).  Against
+// FP64 over |z| < 12: tanh 1.8e-8 rms (2.2e-8 before), squareplus and both
+// derivatives unchanged, softplus 4.5e-8 (3.9e-8) and its derivative 4.8e-8
+// (4.6e-8) with half the bias.  Polynomials are Chebyshev fits of the named
+// function, made for this range.
+__device__ __forceinline__ float mlp_act(int actfn, float z, float &d) {
   switch (actfn) {
     case 0:
       d = z > 0.f ? 1.f : 0.f;
       return z > 0.f ? z : 0.f;
     case 1: {
-      float ex = expf(z);
-      const float thr = -13.942385152878742f;  // log(FLT_EPSILON) + 2
-      d = 1.f / (1.f + 1.f / ex);
-      return z < -thr ? log1pf(ex) : z;
+      // softplus = max(z, 0) + log1p(a), a = exp(-|z|);
+      // log1p(a) = 2 atanh(s), s = a / (2 + a) <= 1/3
+      const float a = expf(-fabsf(z));
+      const float u = 1.f + a, r = mlp_rcp(u);
+      d = z >= 0.f ? r : mlp_div(a, u, r);
+      const float v = 2.f + a, rv = mlp_rcp(v);
+      float s = mlp_div(a, v, rv);
+      s = fmaf(-s * (a - (v - 2.f)), rv, s);  // v's rounding
+      const float s2 = s * s;
+      // (atanh(s)/s - 1)/s^2
+      float p = fmaf(0.11619523f, s2, 0.10851658f);
+      p = fmaf(p, s2, 0.14296292f);
+      p = fmaf(p, s2, 0.19999851f);
+      p = fmaf(p, s2, 0.33333334f);
+      return fmaf(2.f, fmaf(s * s2, p, s), z >= 0.f ? z : 0.f);
     }
     case 2: {
       // tanh' = sech^2 z = 4 e / (1 + e)^2 with e = exp(-2|z|): the same
       // value as 1 - tanh^2, without its cancellation (at |z| = 3 one ulp
       // of tanh is 1e-5 of 1 - tanh^2, an error that does not cancel in the
-      // virial)
-      const float e = expf(-2.f * fabsf(z));
-      const float u = 1.f + e;
-      d = 4.f * e / (u * u);
-      return tanhf(z);
+      // virial).  tanh = 1 - 2 e / (1 + e), and near 0, where that cancels,
+      // z + z^3 p(z^2)
+      const float t = fabsf(z);
+      const float e = expf(-2.f * t);
+      const float u = 1.f + e, r = mlp_rcp(u);
+      d = mlp_div(4.f * e, u * u, r * r);
+      const float s = z * z;
+      // (tanh(z)/z - 1)/z^2 on |z| < 0.55
+      float p = fmaf(-0.0066157525f, s, 0.021312743f);
+      p = fmaf(p, s, -0.053910066f);
+      p = fmaf(p, s, 0.13333118f);
+      p = fmaf(p, s, -0.33333332f);
+      const float small = fmaf(t * s, p, t), large = fmaf(-2.f * e, r, 1.f);
+      return copysignf(t < 0.55f ? small : large, z);
     }
     default: {
       // squareplus 0.5 (z + sqrt(z^2 + 4)); for z < 0 the same value is
       // 2 / (sqrt(z^2 + 4) - z), which avoids the cancellation that costs
       // FP32 most of its digits when z << 0
-      float q = sqrtf(z * z + 4.f);
-      float y = z >= 0.f ? 0.5f * (z + q) : 2.f / (q - z);
-      d = y / q;
+      const float w = fmaf(z, z, 4.f);
+      float i;
+      asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(i) : "f"(w));
+      const float q0 = w * i;
+      const float q = fmaf(fmaf(-q0, q0, w), 0.5f * i, q0);
+      const float iq = fmaf(i, fmaf(-q, i, 1.f), i);
+      const float v = q - z;
+      const float y = z >= 0.f ? 0.5f * (z + q) : mlp_div(2.f, v, mlp_rcp(v));
+      d = mlp_div(y, q, iq);
       return y;
     }
   }

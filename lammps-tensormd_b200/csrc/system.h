@@ -103,7 +103,7 @@ struct tmd_system {
   // kernel form of the pair-force loop (kForce*), set by the default rule,
   // tmd_system_set_variant or tmd_system_autotune
   int force_variant = 0;
-  int desc_variant = 0;    // kDesc*, the same way
+  int desc_variant = -1;     // kDesc*, the same way; -1: the library chooses (desc_form)
   long long wait_probe = 0;  // tmd_system_set_wait_probe (failure-detection tests)
   // temperature-dependent model: electron temperature (eV), per-atom
   // entropy and free energy, and their totals of the last compute
@@ -187,7 +187,6 @@ int rebuild_now(tmd_system *s);
 void launch_force_eval(tmd_system *s, float scale, bool want_vatom);
 ForceArgs force_args(tmd_system *s, float scale, int variant);
 DescArgs desc_args(tmd_system *s, int variant);
-int default_desc_variant(const tmd_model *m);
 // Kernel form of the force loop used when nothing chose one.
 int default_force_variant(const tmd_model *m);
 NbArgs nb_args(tmd_system *s);
