@@ -1246,11 +1246,11 @@ int tmd_system_create(const tmd_model *m, int natoms_cap, double skin,
   A(P, N * h.nelt * h.K * basis_count(h.D)); A(G, N * h.nin); A(dEdG, N * h.nin); A(E, N);
   A(wv, 6 * N); A(eatom, N); A(vatom, 6 * N); A(ke, N);
   if (h.tdnp) { A(tdnp_s, N); A(tdnp_a, N); A(tdnp_tot, 2); }
-  A(partial, 1024 * 8); A(scal, 8);
+  A(partial, 1024 * 8); A(scal, 10);
   A(flag, 2); A(status, 2);  // flag[0] rebuild pending, flag[1] rebuilds done
   A(perm, N); A(tiles, 3 * (N / (m->mlp_tr > 0 ? m->mlp_tr : m->mlp.form[0].rows) + h.nelt + 1));
 #undef A
-  if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void **>(&s->h_scal), 8 * sizeof(double));
+  if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void **>(&s->h_scal), 10 * sizeof(double));
   if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void **>(&s->h_status), 4 * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(s->v, 0, 3 * N * sizeof(double));
   if (e == cudaSuccess) e = cudaMemset(s->image, 0, 3 * N * sizeof(int));
@@ -1464,21 +1464,17 @@ int tmd_compute(tmd_system *s, int eflag, int vflag, double scale, double *energ
   // forces and per-atom virials to every atom, ghosts included
   const int nl = n - s->nghost;
   launch_force_eval(s, (float)scale, want_vatom);
-  if (eflag || energy)
-    launch_reduce_scaled(s->E, nl, s->partial, s->scal, scale, s->st, s->launches);
   if (s->m->h.tdnp) {
     // entropy and free energy totals of the temperature-dependent model
     // (TensorMD::run, tensormd.cpp:491-492: S and A times the pair scale)
     launch_reduce_scaled(s->tdnp_s, nl, s->partial, s->tdnp_tot, scale, s->st, s->launches);
     launch_reduce_scaled(s->tdnp_a, nl, s->partial, s->tdnp_tot + 1, scale, s->st, s->launches);
   }
-  if (vflag || virial)
-    launch_reduce_f64(s->wv, nl, 6, s->partial, s->scal + 1, s->st, s->launches);
-  launch_check_finite(n, s->f, (eflag || energy) ? s->scal : nullptr, s->status, s->st,
-                      s->launches);
+  launch_results((eflag || energy) ? s->E : nullptr, (vflag || virial) ? s->wv : nullptr, nl, s->f,
+                 n, scale, s->partial, s->status, s->flag, s->scal, s->st, s->launches);
   TMD_CUDA(cudaGetLastError());
   if (eatom && nl > 0) launch_scale_copy(s->E, nl, scale, s->eatom, s->st, s->launches);
-  TMD_CUDA(cudaMemcpyAsync(s->h_scal, s->scal, 7 * sizeof(double), cudaMemcpyDeviceToHost, s->st));
+  TMD_CUDA(cudaMemcpyAsync(s->h_scal, s->scal, 10 * sizeof(double), cudaMemcpyDeviceToHost, s->st));
   if (f) TMD_CUDA(cudaMemcpyAsync(f, s->f, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, s->st));
   if (eatom) {
     if (nl > 0)
@@ -1486,8 +1482,9 @@ int tmd_compute(tmd_system *s, int eflag, int vflag, double scale, double *energ
     for (int i = nl; i < n; i++) eatom[i] = 0.0;  // ghosts carry no energy
   }
   if (vatom) TMD_CUDA(cudaMemcpyAsync(vatom, s->vatom, 6 * n * sizeof(double), cudaMemcpyDeviceToHost, s->st));
-  rc = read_status(s);
-  if (rc) return rc;
+  TMD_CUDA(cudaStreamSynchronize(s->st));
+  std::memcpy(s->h_status, s->h_scal + 8, 3 * sizeof(int));
+  account_pos_rebuilds(s, s->h_status[2]);
   int st = s->h_status[0];
   if (st & kStatusOverflow) {
     // positions moved enough to overflow the list: rebuild larger and redo

@@ -291,6 +291,72 @@ __global__ void k_check_finite(int n, const double *__restrict__ f,
   if (bad) atomicOr(status, kStatusNonfinite);
 }
 
+// Totals of a force evaluation in two launches: FP64 sums of E (times scale)
+// and of the virial rows, and the finiteness of the forces; the final block
+// also hands over and clears the status words, so that the host reads one
+// 80-byte record.  Sum order as launch_reduce_scaled / launch_reduce_f64.
+// Separate reductions, check, status copies and clear were nine stream
+// operations at the end of every tmd_compute, here three.
+__global__ void k_result_partial(const double *__restrict__ E, const double *__restrict__ wv,
+                                 int nl, const double *__restrict__ f, int n, double scale,
+                                 double *__restrict__ partial, int *status) {
+  __shared__ double sh[kRedThreads];
+  const int per = (nl + gridDim.x - 1) / gridDim.x;
+  const int i0 = blockIdx.x * per, i1 = min(nl, i0 + per);
+  double s[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    if (E) s[0] += E[i];
+    if (wv)
+#pragma unroll
+      for (int c = 0; c < 6; c++) s[1 + c] += wv[(size_t)i * 6 + c];
+  }
+  for (int c = 0; c < 7; c++) {
+    if (c == 0 ? E == nullptr : wv == nullptr) continue;
+    const double t = block_sum(s[c], sh);
+    if (threadIdx.x == 0) partial[(size_t)blockIdx.x * 7 + c] = c == 0 ? t * scale : t;
+  }
+  bool bad = false;
+  for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < 3L * n;
+       k += (long)gridDim.x * blockDim.x)
+    bad |= !isfinite(f[k]);
+  if (bad) atomicOr(status, kStatusNonfinite);
+}
+
+__global__ void k_result_final(const double *__restrict__ partial, int nb, bool want_e,
+                               bool want_v, int *status, const int *flag,
+                               double *__restrict__ out) {
+  __shared__ double sh[kRedThreads];
+  bool bad = false;
+  for (int c = 0; c < 7; c++) {
+    if (c == 0 ? !want_e : !want_v) continue;
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) s += partial[(size_t)b * 7 + c];
+    s = block_sum(s, sh);
+    if (threadIdx.x == 0) {
+      out[c] = s;
+      if (c == 0 && !isfinite(s)) bad = true;
+    }
+  }
+  if (threadIdx.x == 0) {
+    int *w = reinterpret_cast<int *>(out + 8);
+    w[0] = status[0] | (bad ? kStatusNonfinite : 0);
+    w[1] = status[1];
+    w[2] = flag[1];
+    status[0] = 0;
+    status[1] = 0;
+  }
+}
+
+void launch_results(const double *E, const double *wv, int nl, const double *f, int n,
+                    double scale, double *partial, int *status, const int *flag, double *out,
+                    cudaStream_t st, long &launches) {
+  const int nb = red_blocks(nl);
+  k_result_partial<<<nb, kRedThreads, 0, st>>>(E, wv, nl, f, n, scale, partial, status);
+  k_result_final<<<1, kRedThreads, 0, st>>>(partial, nb, E != nullptr, wv != nullptr, status,
+                                           flag, out);
+  launches += 2;
+}
+
 void launch_check_finite(int n, const double *f, const double *etot, int *status,
                          cudaStream_t st, long &launches) {
   int grid = (n + 255) / 256;

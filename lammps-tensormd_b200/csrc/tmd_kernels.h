@@ -73,7 +73,7 @@ void launch_rebuild_cond(cudaGraphConditionalHandle h, const int *flag, cudaStre
 void launch_nearest_image(int n, double *x, const double *xbuild, const BoxP &box,
                           const BoxP *cbox, const int *acell, cudaStream_t st, long &launches);
 
-// Descriptor: P[n][B][K][D], G[n][B*K*M].
+// Descriptor: P[n][B][K][E] (E = basis_count(D)), G[n][B*K*M].
 // Kernel forms: K/4 lanes per atom with 4 filters each (k_descriptor), or
 // min(K, 32) lanes per atom with K/min(K, 32) filters each and the monomials
 // of each pair computed once (k_descriptor_w).
@@ -272,7 +272,7 @@ struct ForceArgs {
   const uint32_t *nbr;
   const int *boff;
   // S = dE/dP is formed per (atom, block) from the descriptor moments P
-  // [n][B][K][D] and the MLP rows G, dE/dG [n*B*K][M] (dedp_row)
+  // [n][B][K][E] and the MLP rows G, dE/dG [n*B*K][M] (dedp_row)
   const float *P, *G, *dEdG;
   float4 *pdf;
   double *wv;  // [n][6] per-atom sum of -r_ij (x) df over own pairs
@@ -305,6 +305,13 @@ void launch_gather(const GatherArgs &a, cudaStream_t st, long &launches);
 // FP32 input).  partial has >= 1024*ncomp doubles.
 void launch_reduce_f64(const double *in, int n, int ncomp, double *partial,
                        double *out, cudaStream_t st, long &launches);
+// Totals of a force evaluation: out[0] = scale * sum E, out[1..6] = sums of the
+// virial rows wv[nl][6] (E or wv null: skipped), non-finite forces f[n][3] or
+// energy into status; out + 8 as int[3]: status[0], status[1] (both then
+// cleared) and flag[1].  partial has >= 1024*7 doubles.
+void launch_results(const double *E, const double *wv, int nl, const double *f, int n,
+                    double scale, double *partial, int *status, const int *flag, double *out,
+                    cudaStream_t st, long &launches);
 void launch_reduce_scaled(const double *in, int n, double *partial, double *out,
                           double scale, cudaStream_t st, long &launches);
 // Per-cell sums in a fixed order: out[c*ostride + k] = scale * sum over the
