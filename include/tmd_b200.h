@@ -235,7 +235,8 @@ int tmd_system_tdnp_energies(tmd_system *sys, double *entropy, double *free_ener
  * of their mbarriers, before any MMA or copy is issued; nothing arrives on
  * it, so each CTA takes its timeout path (no asynchronous work in flight,
  * TMEM freed) and tmd_compute returns TMD_ERR_TIMEOUT with the context still
- * usable.  cycles = 0 (the default) turns it off; the FP32 MLP has no waits. */
+ * usable.  cycles = 0 (the default) turns it off; the FP32 MLP's bounded
+ * waits (copies of its weight stream) are not probed. */
 int tmd_system_set_wait_probe(tmd_system *sys, long long cycles);
 
 /* Measured FP32 issue peak of a device: a packed-FMA (FFMA2) kernel with
