@@ -208,8 +208,8 @@ __device__ inline PairGeo load_pair_geo(const float4 *__restrict__ src, int &t) 
 
 // P_0 = sum_j H_k, by far the largest of a filter's sums and the one whose
 // rounding reaches G_0 and G_2 together, is summed in runs of 16 pairs: a run
-// starts from zero and is folded into p0 at its end (the same runs in every
-// one-stream form, so their sums agree bit for bit).  On BCC
+// starts from zero and is folded into p0 at its end (the same runs in the wide
+// and the split form, whose sums agree bit for bit).  On BCC
 // cells this takes the descriptor's share of the force error from 2.8e-6 (one
 // running sum, 20 monomials) to 1.7e-6.
 template <int F, int N>
@@ -386,30 +386,30 @@ k_descriptor_w(KParams kp, BoxP box, int n, int cap, const double *__restrict__ 
       nact += cnt;
       constexpr int kRun = W < 16 ? W : 16;
       for (int h = 0; h < cnt; h += kRun) {
-      const int ce = min(cnt, h + kRun);
+        const int ce = min(cnt, h + kRun);
 #pragma unroll kPairUnroll<RK>
-      for (int c = h; c < ce; c++) {
-        const PairGeo g = geo_load_radial<RK>(pr.slot(c));
-        const float4 *ms = reinterpret_cast<const float4 *>(
-            mr + ((pr.head + c) & (PairRing<W>::kSlots - 1)) * D4);
-        float2 h2[FPL];
-#pragma unroll
-        for (int f = 0; f < FPL; f++) {
-          const float h = radial1<RK>(kp, R[f], g);
-          h2[f] = make_float2(h, h);
-        }
-#pragma unroll
-        for (int v = 0; v < D4 / 4; v++) {
-          const float4 m4 = ms[v];
-          const float2 lo = make_float2(m4.x, m4.y), hi = make_float2(m4.z, m4.w);
+        for (int c = h; c < ce; c++) {
+          const PairGeo g = geo_load_radial<RK>(pr.slot(c));
+          const float4 *ms = reinterpret_cast<const float4 *>(
+              mr + ((pr.head + c) & (PairRing<W>::kSlots - 1)) * D4);
+          float2 h2[FPL];
 #pragma unroll
           for (int f = 0; f < FPL; f++) {
-            acc[f][2 * v] = __ffma2_rn(h2[f], lo, acc[f][2 * v]);
-            acc[f][2 * v + 1] = __ffma2_rn(h2[f], hi, acc[f][2 * v + 1]);
+            const float h = radial1<RK>(kp, R[f], g);
+            h2[f] = make_float2(h, h);
+          }
+#pragma unroll
+          for (int v = 0; v < D4 / 4; v++) {
+            const float4 m4 = ms[v];
+            const float2 lo = make_float2(m4.x, m4.y), hi = make_float2(m4.z, m4.w);
+#pragma unroll
+            for (int f = 0; f < FPL; f++) {
+              acc[f][2 * v] = __ffma2_rn(h2[f], lo, acc[f][2 * v]);
+              acc[f][2 * v + 1] = __ffma2_rn(h2[f], hi, acc[f][2 * v + 1]);
+            }
           }
         }
-      }
-      if (((nact - cnt - nact0 + ce) & 15) == 0) fold_p0(acc, p0);
+        if (((nact - cnt - nact0 + ce) & 15) == 0) fold_p0(acc, p0);
       }
       pr.pop(cnt);
     }
@@ -729,38 +729,38 @@ k_descriptor_c(KParams kp, int n, int cap, float *__restrict__ P, float *__restr
       const float *cs = sg + buf * W * SL;
       constexpr int kRun = W < 16 ? W : 16;
       for (int h = 0; h < cnt; h += kRun) {
-      const int ce = min(cnt, h + kRun);
+        const int ce = min(cnt, h + kRun);
 #pragma unroll kPairUnroll<RK>
-      for (int c = h; c < ce; c++) {
-        const float4 *ms = reinterpret_cast<const float4 *>(cs + c * SL);
-        const float4 rr = ms[D4 / 4];
-        PairGeo g;
-        g.ux = g.uy = g.uz = g.dfc = g.rinv = 0.f;
-        if (RK == kRadTable) {
-          g.r = g.rlo = g.fc = 0.f;
-          g.tq = rr.z;
-          g.ti = __float_as_int(rr.w);
-        } else {
-          g.r = rr.x; g.rlo = rr.y; g.fc = rr.z; g.tq = 0.f; g.ti = 0;
-        }
-        float2 h2[FPL];
-#pragma unroll
-        for (int f = 0; f < FPL; f++) {
-          const float h = radial1<RK>(kp, R[f], g);
-          h2[f] = make_float2(h, h);
-        }
-#pragma unroll
-        for (int v = 0; v < D4 / 4; v++) {
-          const float4 m4 = ms[v];
-          const float2 lo = make_float2(m4.x, m4.y), hi = make_float2(m4.z, m4.w);
+        for (int c = h; c < ce; c++) {
+          const float4 *ms = reinterpret_cast<const float4 *>(cs + c * SL);
+          const float4 rr = ms[D4 / 4];
+          PairGeo g;
+          g.ux = g.uy = g.uz = g.dfc = g.rinv = 0.f;
+          if (RK == kRadTable) {
+            g.r = g.rlo = g.fc = 0.f;
+            g.tq = rr.z;
+            g.ti = __float_as_int(rr.w);
+          } else {
+            g.r = rr.x; g.rlo = rr.y; g.fc = rr.z; g.tq = 0.f; g.ti = 0;
+          }
+          float2 h2[FPL];
 #pragma unroll
           for (int f = 0; f < FPL; f++) {
-            acc[f][2 * v] = __ffma2_rn(h2[f], lo, acc[f][2 * v]);
-            acc[f][2 * v + 1] = __ffma2_rn(h2[f], hi, acc[f][2 * v + 1]);
+            const float h = radial1<RK>(kp, R[f], g);
+            h2[f] = make_float2(h, h);
+          }
+#pragma unroll
+          for (int v = 0; v < D4 / 4; v++) {
+            const float4 m4 = ms[v];
+            const float2 lo = make_float2(m4.x, m4.y), hi = make_float2(m4.z, m4.w);
+#pragma unroll
+            for (int f = 0; f < FPL; f++) {
+              acc[f][2 * v] = __ffma2_rn(h2[f], lo, acc[f][2 * v]);
+              acc[f][2 * v + 1] = __ffma2_rn(h2[f], hi, acc[f][2 * v + 1]);
+            }
           }
         }
-      }
-      if (((c0 + ce) & 15) == 0) fold_p0(acc, p0);
+        if (((c0 + ce) & 15) == 0) fold_p0(acc, p0);
       }
       buf ^= 1;
     }

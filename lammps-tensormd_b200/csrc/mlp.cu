@@ -71,7 +71,7 @@ int mlp_fp32_form(const MlpPlan &p, const int *count, int nelt) {
   // atoms 15.7 / 12.7 / 23 / 32 us, 23,040 atoms of a 128-wide net - / 231 /
   // 151 / 143, 128,000 atoms - / 196 / 145 / 155, 1,048,576 atoms - / 2087 /
   // 1673 / 1506.
-  static const double lat[4] = {10.0, 13.6, 25.0, 37.0}, thr[4] = {7.0, 7.4, 10.0, 18.0};
+  static const double lat[4] = {10.0, 13.6, 25.0, 37.0}, thr[4] = {7.0, 7.4, 10.0, 19.4};
   int best = -1;
   double best_c = 0.0;
   for (int v = 0; v < 4; v++) {
