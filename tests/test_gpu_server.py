@@ -7,9 +7,10 @@
   NVE jobs           nsteps run; end state bitwise that of tmd_nve_run of the
                      same system (energy sums to 1e-12 relative)
   FIRE jobs          LAMMPS min_style fire (its defaults) against the FP64
-                     oracle's restatement of min_fire.cpp: a 200-iteration
-                     trajectory on a random-weight potential (positions
-                     within 1e-4 A, energy 1e-6 eV/atom), and a relaxation on
+                     oracle's restatement of min_fire.cpp: trajectories of 90
+                     and 200 iterations on a random-weight potential, from
+                     starts where they are stable (positions within 1e-4 A,
+                     energy 1e-6 eV/atom), and a relaxation on
                      the trained MoNi potential to max |F_i| < 0.01 eV/A in
                      the oracle's number of iterations
   concurrency        mixed jobs from several threads all complete; results
@@ -25,7 +26,8 @@ import numpy as np
 import pytest
 
 from pack import Oracle, load_npz
-from tmd_testutil import GOLDEN, frac_wrap, read_data
+from tmd_testutil import (FIRE_STARTS, GOLDEN, cell_distance, fire_potential, fire_start,
+                          frac_wrap, read_data)
 from tmd_b200 import TensorMDModel, TensorMDServer, TensorMDSystem, TmdError, synth
 
 pytestmark = pytest.mark.gpu
@@ -34,8 +36,7 @@ pytestmark = pytest.mark.gpu
 @pytest.fixture(scope="module")
 def model4(tmp_path_factory):
     p = tmp_path_factory.mktemp("pot") / "serve.npz"
-    syms = synth.gaussian_potential(p, seed=31, nelt=4, num_filters=16, rc=6.0,
-                                    max_moment=3, hidden=(64, 64), actfn=2)
+    syms = fire_potential(p)
     m = TensorMDModel(f"{p} {' '.join(syms)}")
     m.npz_path = str(p)
     return m
@@ -217,23 +218,20 @@ def test_fire_job_converges_as_the_oracle():
     np.testing.assert_allclose(ref["f"], out["f"], rtol=0, atol=1e-6)
 
 
-def test_fire_trajectory_follows_the_oracle(model4):
-    """200 FIRE iterations of a 64-atom amorphous cell in the server against
-    the FP64 oracle's min_style fire (same defaults, same start, v = 0):
-    every P = F.v sign, step back and dt change must agree for the end
-    positions to agree."""
-    rng = np.random.default_rng(21)
-    x, box = synth.random_packing(64, rng)
-    t = rng.integers(1, 5, size=64).astype(np.int32)
+@pytest.mark.parametrize("seed,steps", FIRE_STARTS)
+def test_fire_trajectory_follows_the_oracle(model4, seed, steps):
+    """FIRE iterations of a 64-atom amorphous cell in the server against the
+    FP64 oracle's min_style fire (same defaults, same start, v = 0): every
+    P = F.v sign, step back and dt change must agree for the end positions to
+    agree.  The starts are stable ones, so that FP32 rounding decides no branch."""
+    x, t, box = fire_start(seed)
     srv = TensorMDServer(model4, max_atoms=10000, max_cells=8, steps_per_tick=16)
-    out = srv.wait(srv.submit(2, x, t, box, nsteps=200, dt=0.001, fmax=1e-9), timeout=300)
+    out = srv.wait(srv.submit(2, x, t, box, nsteps=steps, dt=0.001, fmax=1e-9), timeout=300)
     srv.close()
     o = Oracle(load_npz(model4.npz_path))
-    xo, fo, eo, it = o.fire(x, t - 1, box, [1, 1, 1], 0.001, 1e-9, 200)
-    assert out["steps"] == it == 200
-    L = box[3:6]
-    d = (out["x"] - xo) - np.round((out["x"] - xo) / L) * L
-    assert np.abs(d).max() < 1e-4, np.abs(d).max()
+    xo, fo, eo, it = o.fire(x, t - 1, box, [1, 1, 1], 0.001, 1e-9, steps)
+    assert out["steps"] == it == steps
+    assert cell_distance(out["x"], xo, box) < 1e-4, cell_distance(out["x"], xo, box)
     assert abs(out["energy"] - eo) / len(x) < 1e-6
     assert eo < o.compute(x, t - 1, box, [1, 1, 1])["energy"]
 

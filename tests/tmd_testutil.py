@@ -13,6 +13,34 @@ GOLDEN = ROOT / "tests" / "golden"
 NKTV2P = 1.6021765e6  # metal units, update.cpp:187-206
 
 
+# FIRE starts (seed of a 64-atom packing, iterations) whose trajectories are
+# stable: the FP64 oracle, started 1e-7 A away, stays within 2e-4 A of its own
+# (test_fire_starts.py).  Most packings come near a zero of the power F.v
+# within 200 iterations, and a 1e-8 A change of the start then flips a branch;
+# these do not, or (90 iterations) end before they do.
+FIRE_STARTS = [(23, 200), (26, 200), (21, 90), (28, 90)]
+
+
+def fire_start(seed):
+    from tmd_b200 import synth
+    rng = np.random.default_rng(seed)
+    x, box = synth.random_packing(64, rng)
+    return x, rng.integers(1, 5, size=64).astype(np.int32), box
+
+
+def fire_potential(path):
+    """The four-element random-weight potential of the serving tests."""
+    from tmd_b200 import synth
+    return synth.gaussian_potential(path, seed=31, nelt=4, num_filters=16, rc=6.0, max_moment=3,
+                                    hidden=(64, 64), actfn=2)
+
+
+def cell_distance(a, b, box):
+    """Largest coordinate difference of two configurations of an orthogonal cell."""
+    d = a - b
+    return float(np.abs(d - np.round(d / box[3:6]) * box[3:6]).max())
+
+
 def published():
     return json.loads((GOLDEN / "published.json").read_text())
 
