@@ -197,7 +197,7 @@ __device__ inline PairGeo decode_pair_geo(const float4 a, const float4 b, int &t
     g.fc = b.y; g.dfc = b.z; g.ti = 0; g.tq = 0.f;
   }
   t = __float_as_int(b.w);
-  g.rinv = rcp_newton(g.r);
+  g.rinv = rcp_sum(g.r, g.rlo);  // as pair_geometry
   return g;
 }
 

@@ -7,6 +7,7 @@
 // xyy, xyz, xzz, yyy, yyz, yzz, zzz.
 #pragma once
 
+#include "rcp.cuh"
 #include "tmd_internal.h"
 
 namespace tmd {
@@ -17,7 +18,7 @@ struct PairGeo {
   float ux, uy, uz;     // unit vector (x_j - x_i) / r
   float fc, dfc;        // analytic cutoff and derivative
   float tq;             // table: offset inside the interval
-  float rinv;           // 1 / r (FP32)
+  float rinv;           // 1 / (r + rlo)
   int ti;               // table interval (0 for analytic), -1 when inactive
 };
 
@@ -48,41 +49,15 @@ __device__ inline NbPos load_nb(const double *__restrict__ x, uint32_t e, bool v
   return p;
 }
 
-// sin and cos of pi t for |t| <= 1/2 (odd and even Chebyshev fits made for
-// this range, absolute errors 7e-9 and 2e-10).
-__device__ __forceinline__ void sincospi_half(float t, float &s, float &c) {
-  const float q = t * t;
-  float p = fmaf(0.07765766f, q, -0.59829129f);
-  p = fmaf(p, q, 2.55007752f);
-  p = fmaf(p, q, -5.16771008f);
-  s = fmaf(t, fmaf(p, q, 3.14159274f), t * -1.0033e-7f);  // the fit's 3.1415926401 in two parts
-  p = fmaf(-0.02439632f, q, 0.23493731f);
-  p = fmaf(p, q, -1.33521200f);
-  p = fmaf(p, q, 4.05870916f);
-  p = fmaf(p, q, -4.93480214f);
-  c = fmaf(p, q, 1.f);
-}
-
-// 1/x to about half an ulp for normal x (approximate reciprocal, one Newton
-// step; no range handling).
-__device__ __forceinline__ float rcp_newton(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return fmaf(r, fmaf(-x, r, 1.f), r);
-}
-
 // Geometry of one pair (FP64 difference and cutoff test rij2 < rc^2 &&
 // rij2 > 1e-10 as kernel.cu:1163).  g.ti = -1 if inactive.
+// 1/r is that of r + rlo.  The shift is decoded for image entries only.
 //
-// The distance comes from an FP32 reciprocal square root and one FP64
-// correction: rf = r2 / sqrt(r2) in FP32, r2 - rf^2 exactly in FP64, and the
-// Newton term of that in FP32 as the low part, renormalised so that r is the
-// nearest FP32 value; r + rlo holds the FP64 root to 3e-14 relative.  With the
-// cutoff's sine and cosine as two polynomials and the shift decoded only for
-// image entries, k_pair_geo takes 97 M instead of 127 M warp instructions at
-// 128,000 atoms (FP64 sqrt, IEEE divide and sincospif before; it is bound by
-// its scattered loads, 192 -> 183 us) and the fused descriptor 4.21 -> 4.06 ms
-// on 4,096 cells.
+// The root, the cutoff's sine and cosine are the plain functions: an FP32
+// root with one correction and polynomials of absolute accuracy gave 7 of
+// 410 us of the fused descriptor at 128,000 atoms, and cost the relative
+// accuracy of f_c and f_c' near rc (forces of rank-3 dimers at 0.98 to 0.998
+// rc 2.6e-5 off, against 1.0e-5).
 __device__ inline void pair_geometry(const KParams &kp, const BoxP &box, double xi,
                                      double yi, double zi, const NbPos &p,
                                      PairGeo &g) {
@@ -99,22 +74,15 @@ __device__ inline void pair_geometry(const KParams &kp, const BoxP &box, double 
   const double dx = gx - xi, dy = gy - yi, dz = gz - zi;
   const double r2 = rsq_plain(dx, dy, dz);
   if (!(r2 < kp.rcsq && r2 > 1e-10)) return;
-  const float r2f = float(r2);
-  float ri;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ri) : "f"(r2f));
-  const float ra = r2f * ri;
-  const float lo = 0.5f * ri * float(fma(-double(ra), double(ra), r2));
-  const float rf = ra + lo;
-  const float rinv = fmaf(ri, fmaf(-rf, ri, 1.f), ri);
+  const double r = sqrt(r2);
+  const float rf = float(r);
   g.r = rf;
-  g.rinv = rinv;
-  g.rlo = lo - (rf - ra);
-  const float ru = fmaf(-rinv * rinv, g.rlo, rinv);  // 1 / (r + rlo)
-  g.ux = float(dx) * ru;
-  g.uy = float(dy) * ru;
-  g.uz = float(dz) * ru;
+  g.rlo = float(r - double(rf));
+  g.rinv = rcp_sum(rf, g.rlo);
+  g.ux = float(dx) * g.rinv;
+  g.uy = float(dy) * g.rinv;
+  g.uz = float(dz) * g.rinv;
   if (kp.radial == 1) {
-    const double r = double(rf) + double(g.rlo);
     int ti = int(r * kp.tab_xdxd);
     if (ti > kp.tab_n - 2) ti = kp.tab_n - 2;
     g.ti = ti;
@@ -123,11 +91,11 @@ __device__ inline void pair_geometry(const KParams &kp, const BoxP &box, double 
     g.ti = 0;
     float z = rf * kp.inv_rc;
     if (kp.fctype == 0) {
-      // cos(pi z) = -sin(pi (z - 1/2)), sin(pi z) = cos(pi (z - 1/2))
+      z = z > 1.f ? 1.f : z;
       float s, c;
-      sincospi_half(fminf(z, 1.f) - 0.5f, s, c);
-      g.fc = fmaf(-0.5f, s, 0.5f);
-      g.dfc = -0.5f * 3.14159265358979f * c * kp.inv_rc;
+      sincospif(z, &s, &c);
+      g.fc = 0.5f + 0.5f * c;
+      g.dfc = -0.5f * 3.14159265358979f * s * kp.inv_rc;
     } else {
       const float gm = 5.f;
       z = z > 3.14159265358979f ? 3.14159265358979f : z;
