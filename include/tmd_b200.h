@@ -246,6 +246,12 @@ int tmd_system_set_wait_probe(tmd_system *sys, long long cycles);
  * Uses its own stream and returns after it has finished. */
 int tmd_fp32_peak(int device, int reps, double *tflops);
 
+/* The FP32 MLP's activation `actfn` (0 ReLU, 1 softplus, 2 tanh, 3 squareplus)
+ * and its derivative at n host values z, evaluated on the device by the
+ * function the MLP kernel uses: y[n], d[n] on the host.  For tests of its
+ * accuracy; no reference counterpart.  Returns after it has finished. */
+int tmd_mlp_activation(int device, int actfn, int n, const float *z, float *y, float *d);
+
 /* Kernel timing (TensorMDTimer's phase report, tensormd_timer.h:25-46, with
  * CUDA events instead of host clocks).  enable != 0 records an event pair
  * around every kernel family on the system stream during tmd_compute and

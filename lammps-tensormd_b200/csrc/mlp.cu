@@ -1,11 +1,15 @@
 // mlp.cu -- FP32 MLP: shape limits, forms, weight packing and dispatch
 // (kernel and semantics in mlp_impl.cuh).
 #include <algorithm>
+#include <string>
 #include <vector>
 
 #include "mlp_impl.cuh"
+#include "tmd_b200.h"
 
 namespace tmd {
+
+void set_last_error(const std::string &m);  // abi.cpp
 
 // one object per column-block width (mlp_nt32.cu, mlp_nt64.cu, mlp_nt128.cu)
 extern template void mlp_plan_nt<32>(int, const int *, int, MlpPlan &);
@@ -16,6 +20,15 @@ extern template void launch_mlp_tr<64>(const MlpArgs &, cudaStream_t);
 extern template void launch_mlp_tr<128>(const MlpArgs &, cudaStream_t);
 
 namespace {
+
+__global__ void k_mlp_activation(int actfn, int n, const float *__restrict__ z,
+                                 float *__restrict__ y, float *__restrict__ d) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float di;
+  y[i] = mlp_act(actfn, z[i], di);
+  d[i] = di;
+}
 
 // Column-block width of a net: the narrowest of 32, 64, 128 that holds its
 // widest hidden layer in one block (wider layers take several blocks of 128).
@@ -118,3 +131,29 @@ void launch_mlp_fp32(const MlpArgs &a, cudaStream_t st, long &launches) {
 }
 
 }  // namespace tmd
+
+extern "C" int tmd_mlp_activation(int device, int actfn, int n, const float *z, float *y,
+                                  float *d) {
+  if (actfn < 0 || actfn > 3 || n < 1 || !z || !y || !d) {
+    tmd::set_last_error("tmd_mlp_activation: bad argument");
+    return TMD_ERR_ARG;
+  }
+  int prev = 0;
+  cudaGetDevice(&prev);
+  float *buf = nullptr;
+  const size_t bytes = (size_t)n * sizeof(float);
+  cudaError_t e = cudaSetDevice(device);
+  if (e == cudaSuccess) e = cudaMalloc(&buf, 3 * bytes);
+  if (e == cudaSuccess) e = cudaMemcpy(buf, z, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    tmd::k_mlp_activation<<<(n + 255) / 256, 256>>>(actfn, n, buf, buf + n, buf + 2 * (size_t)n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(y, buf + n, bytes, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(d, buf + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost);
+  if (buf) cudaFree(buf);
+  cudaSetDevice(prev);
+  if (e == cudaSuccess) return TMD_OK;
+  tmd::set_last_error(std::string("tmd_mlp_activation: ") + cudaGetErrorString(e));
+  return TMD_ERR_CUDA;
+}

@@ -43,6 +43,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "rcp.cuh"
 #include "tc_util.cuh"
 #include "tmd_kernels.h"
 
@@ -52,83 +53,81 @@ constexpr int kMlpThreads = 128;  // consumers: the threads of the GEMMs and epi
 constexpr int kMlpBlock = kMlpThreads + 32;  // and one producer warp
 constexpr int kMlpPad = 32;  // reduction rows of the packed weights are padded to this
 
-// 1/u and a/u, to about half an ulp, for u between 1 and 2^60: the
-// approximate reciprocal and one Newton step, without the scaling that the
-// full-range division needs.
-__device__ __forceinline__ float mlp_rcp(float u) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(u));
-  return fmaf(r, fmaf(-u, r, 1.f), r);
-}
-__device__ __forceinline__ float mlp_div(float a, float u, float rcp_u) {
-  const float q = a * rcp_u;
-  return fmaf(fmaf(-q, u, a), rcp_u, q);
+// x < lim ? a : b as one select.  Left to the compiler, the cheaper side's
+// operands go behind a branch that diverges lane by lane.
+__device__ __forceinline__ float mlp_select(float x, float lim, float a, float b) {
+  float y;
+  asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %3, %4;\n\tselp.f32 %0, %1, %2, p;\n\t}"
+      : "=f"(y)
+      : "f"(a), "f"(b), "f"(x), "f"(lim));
+  return y;
 }
 
-// Activation and its derivative (nnp.cu:9-57), each from one exponential (or
-// square root) and one or two reciprocals, branch-free: the epilogues were a
-// sixth to a third of the kernel with expf, tanhf or log1pf and IEEE divisions
-// (432,000-atom alloy, softplus: 4.50 -> 3.91 ms; 23,040-atom W net,
-// squareplus: 169 -> 143 us; 128,000 atoms, tanh: 160 -> 145 us).  Against
-// FP64 over |z| < 12: tanh 1.8e-8 rms (2.2e-8 before), squareplus and both
-// derivatives unchanged, softplus 4.5e-8 (3.9e-8) and its derivative 4.8e-8
-// (4.6e-8) with half the bias.  Polynomials are Chebyshev fits of the named
-// function, made for this range.
+// Activation and its derivative (nnp.cu:9-57).  With one or two full-range
+// divisions per value the epilogues were a sixth to a third of the kernel;
+// these take one exponential (or square root) and reciprocals of sums in a
+// known range, three quarters of the time per value (432,000-atom alloy,
+// softplus: 4.50 -> 3.98 ms).  What a sum u = a + b with a >= b loses to
+// rounding is b - (u - a) exactly (Dekker's fast two-sum), so the reciprocals
+// hold the unrounded sum to about half an ulp.  Errors against FP64 over
+// |z| < 12, rms (before, with divisions and tanhf): softplus 3.8e-8 (3.9e-8),
+// its derivative 3.7e-8 (4.6e-8); tanh 1.7e-8 (2.2e-8), 5.4e-8 (7.5e-8);
+// squareplus 3.3e-8 (3.9e-8), 4.8e-8 (5.4e-8).
 __device__ __forceinline__ float mlp_act(int actfn, float z, float &d) {
   switch (actfn) {
     case 0:
       d = z > 0.f ? 1.f : 0.f;
       return z > 0.f ? z : 0.f;
     case 1: {
-      // softplus = max(z, 0) + log1p(a), a = exp(-|z|);
-      // log1p(a) = 2 atanh(s), s = a / (2 + a) <= 1/3
+      // softplus = max(z, 0) + log1p(a), a = exp(-|z|); its derivative is
+      // 1 / (1 + a) or a / (1 + a)
       const float a = expf(-fabsf(z));
-      const float u = 1.f + a, r = mlp_rcp(u);
-      d = z >= 0.f ? r : mlp_div(a, u, r);
-      const float v = 2.f + a, rv = mlp_rcp(v);
-      float s = mlp_div(a, v, rv);
-      s = fmaf(-s * (a - (v - 2.f)), rv, s);  // v's rounding
-      const float s2 = s * s;
-      // (atanh(s)/s - 1)/s^2
-      float p = fmaf(0.11619523f, s2, 0.10851658f);
-      p = fmaf(p, s2, 0.14296292f);
-      p = fmaf(p, s2, 0.19999851f);
-      p = fmaf(p, s2, 0.33333334f);
-      return fmaf(2.f, fmaf(s * s2, p, s), z >= 0.f ? z : 0.f);
+      const float u = 1.f + a, r = rcp_sum(u, a - (u - 1.f));
+      d = mlp_select(z, 0.f, a * r, r);
+      return (z < 0.f ? 0.f : z) + log1pf(a);
     }
     case 2: {
-      // tanh' = sech^2 z = 4 e / (1 + e)^2 with e = exp(-2|z|): the same
-      // value as 1 - tanh^2, without its cancellation (at |z| = 3 one ulp
-      // of tanh is 1e-5 of 1 - tanh^2, an error that does not cancel in the
-      // virial).  tanh = 1 - 2 e / (1 + e), and near 0, where that cancels,
-      // z + z^3 p(z^2)
+      // with e = exp(-2|z|): tanh|z| = 1 - 2 e / (1 + e), whose term loses
+      // (1 - T) / T of an ulp of T = tanh|z| per ulp of its own: half an ulp
+      // and less from T = 2/3, |z| = 0.8.  Below, z + z^3 p(z^2) with p fitted
+      // to that range (3.7e-9 of tanh).  tanh' = 1 - T^2 below and
+      // sech^2 z = 4 e / (1 + e)^2 above, where 1 - T^2 cancels (at |z| = 3
+      // one ulp of T is 1e-5 of it, an error that does not cancel in the
+      // virial).
       const float t = fabsf(z);
       const float e = expf(-2.f * t);
-      const float u = 1.f + e, r = mlp_rcp(u);
-      d = mlp_div(4.f * e, u * u, r * r);
+      const float u = 1.f + e, r = rcp_sum(u, e - (u - 1.f));
       const float s = z * z;
-      // (tanh(z)/z - 1)/z^2 on |z| < 0.55
-      float p = fmaf(-0.0066157525f, s, 0.021312743f);
-      p = fmaf(p, s, -0.053910066f);
-      p = fmaf(p, s, 0.13333118f);
-      p = fmaf(p, s, -0.33333332f);
-      const float small = fmaf(t * s, p, t), large = fmaf(-2.f * e, r, 1.f);
-      return copysignf(t < 0.55f ? small : large, z);
+      float p = fmaf(0.00158704445f, s, -0.00741417659f);
+      p = fmaf(p, s, 0.0213065278f);
+      p = fmaf(p, s, -0.0538535975f);
+      p = fmaf(p, s, 0.133322418f);
+      p = fmaf(p, s, -0.333332986f);
+      const float y = mlp_select(t, 0.8f, fmaf(t * s, p, t), fmaf(-2.f * e, r, 1.f));
+      d = mlp_select(t, 0.8f, fmaf(-y, y, 1.f), 4.f * e * (r * r));
+      return copysignf(y, z);
     }
     default: {
-      // squareplus 0.5 (z + sqrt(z^2 + 4)); for z < 0 the same value is
-      // 2 / (sqrt(z^2 + 4) - z), which avoids the cancellation that costs
-      // FP32 most of its digits when z << 0
+      // squareplus = (z + q) / 2 with q = sqrt(z^2 + 4); for z < 0 the same
+      // value is 2 / (|z| + q), which avoids the cancellation that costs FP32
+      // most of its digits when z << 0.  Derivative: (1 + z / q) / 2, for
+      // z < 0 the value over q.  q and 1/q come from the approximate reciprocal
+      // square root i of w = z^2 + 4 by Karp and Markstein's arrangement of
+      // Newton's step, q = w i + (w - (w i)^2) i / 2 (ACM TOMS 23, 1997), and
+      // a Newton step of 1/q from i.  z is held at -1e18, where the value is
+      // 1e-18 and z^2 does not overflow yet (not-a-number passes); z above
+      // 1.8e19, whose square does, gives not-a-number.
+      asm("max.NaN.f32 %0, %0, 0fDD5E0B6B;" : "+f"(z));
+      const float t = fabsf(z);
       const float w = fmaf(z, z, 4.f);
       float i;
       asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(i) : "f"(w));
       const float q0 = w * i;
       const float q = fmaf(fmaf(-q0, q0, w), 0.5f * i, q0);
       const float iq = fmaf(i, fmaf(-q, i, 1.f), i);
-      const float v = q - z;
-      const float y = z >= 0.f ? 0.5f * (z + q) : mlp_div(2.f, v, mlp_rcp(v));
-      d = mlp_div(y, q, iq);
-      return y;
+      const float v = q + t, n = 2.f * rcp_sum(v, t - (v - q));
+      d = mlp_select(z, 0.f, n * iq, fmaf(0.5f * z, iq, 0.5f));
+      return mlp_select(z, 0.f, n, 0.5f * v);
     }
   }
 }

@@ -17,6 +17,7 @@ ERRORS = {
 # (name, restype, argtypes) for every entry point of include/tmd_b200.h
 _c_int, _c_long, _c_double, _vp = ctypes.c_int, ctypes.c_long, ctypes.c_double, ctypes.c_void_p
 _pd = ctypes.POINTER(ctypes.c_double)
+_pf = ctypes.POINTER(ctypes.c_float)
 _pi = ctypes.POINTER(ctypes.c_int)
 _pl = ctypes.POINTER(ctypes.c_long)
 SIGNATURES = [
@@ -48,6 +49,7 @@ SIGNATURES = [
     ("tmd_system_set_etemp", _c_int, [_vp, _c_double]),
     ("tmd_system_tdnp_energies", _c_int, [_vp, _pd, _pd]),
     ("tmd_fp32_peak", _c_int, [_c_int, _c_int, _pd]),
+    ("tmd_mlp_activation", _c_int, [_c_int, _c_int, _c_int, _pf, _pf, _pf]),
     ("tmd_profile_enable", _c_int, [_vp, _c_int]),
     ("tmd_profile_read", _c_int, [_vp, _pl, _pd, _c_int]),
     ("tmd_last_error", _c_int, [ctypes.c_char_p, _c_int]),
