@@ -958,6 +958,7 @@ int tmd_model_load(const char *coeff_args, int device, tmd_model **out) {
       tmd_model_free(m);
       return fail(TMD_ERR_MODEL, "TDNP nets too wide for the shared-memory work space");
     }
+    mlp_tdnp_prepare();
     m->mlp_tr = 64;  // element grouping only (the TDNP kernel takes atoms directly)
     *out = m;
     return TMD_OK;
@@ -1044,7 +1045,7 @@ int tmd_model_load(const char *coeff_args, int device, tmd_model **out) {
     m->tc_streamed = nsm;
     m->tc_smem_s = ss;
     m->tc_stages = stages;
-    mlp_tcs_prepare(ss, 3, 1, 1);
+    mlp_tcs_prepare(3, 1, 1);
     m->mlp_tr = 128;
   }
   if (h.precision == TMD_PREC_BF16 || h.precision == TMD_PREC_BF16X3 ||
@@ -1141,8 +1142,8 @@ int tmd_model_load(const char *coeff_args, int device, tmd_model **out) {
       return fail(TMD_ERR_CUDA, std::string("tensor-core weight upload: ") +
                                     cudaGetErrorString(e));
     }
-    if (fp8) mlp_fp8_prepare(m->tc_smem, m->tc_dz_bf16);
-    else mlp_tc_prepare(m->tc_smem, m->tc_dz_bf16, np);
+    if (fp8) mlp_fp8_prepare(m->tc_dz_bf16);
+    else mlp_tc_prepare(m->tc_dz_bf16, np);
     // weight-resident persistent form when the hidden weights, one tile's
     // operands and act' fit in shared memory (next to ~3 KB of static data)
     if (!fp8) {
@@ -1163,7 +1164,7 @@ int tmd_model_load(const char *coeff_args, int device, tmd_model **out) {
         m->tc_persistent = 2 * (sp + 4 * 1024) <= 228 * 1024 ? 2 * nsm : nsm;
         m->tc_smem_p = sp;
         m->tc_dz_bf16_p = dzb;
-        mlp_tcp_prepare(sp, np, dzb);
+        mlp_tcp_prepare(np, dzb);
       }
       // weights too large to stay resident: the streamed-weight form, the
       // BF16 form as two CTAs per SM where they fit
@@ -1178,7 +1179,7 @@ int tmd_model_load(const char *coeff_args, int device, tmd_model **out) {
         m->tc_cps = cps;
         m->tc_smem_s = ss;
         m->tc_stages = stages;
-        mlp_tcs_prepare(ss, np, 0, cps);
+        mlp_tcs_prepare(np, 0, cps);
       }
     }
     m->mlp_tr = 128;

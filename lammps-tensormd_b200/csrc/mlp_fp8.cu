@@ -304,10 +304,9 @@ size_t mlp_fp8_smem(int nl, int maxh, int resnet, bool dz_bf16) {
   return b;
 }
 
-void mlp_fp8_prepare(size_t smem, bool dz_bf16) {
-  const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if (dz_bf16) cudaFuncSetAttribute(k_mlp_fp8<__nv_bfloat16>, at, (int)smem);
-  else cudaFuncSetAttribute(k_mlp_fp8<float>, at, (int)smem);
+void mlp_fp8_prepare(bool dz_bf16) {
+  if (dz_bf16) allow_dynamic_smem(k_mlp_fp8<__nv_bfloat16>);
+  else allow_dynamic_smem(k_mlp_fp8<float>);
 }
 
 void launch_mlp_fp8(const MlpTcArgs &a, cudaStream_t st, long &launches) {

@@ -525,7 +525,7 @@ void mlp_plan_one(int nl, const int *sizes, int resnet, MlpPlan &p, int v) {
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return;
     if (f.smem + fa.sharedSizeBytes > 227 * 1024) return;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
+    if (allow_dynamic_smem(kern) != cudaSuccess) return;
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kMlpBlock, f.smem) ==
         cudaSuccess)

@@ -1191,12 +1191,11 @@ int mlp_tcs_hi2(int nl, const int *sizes, int np, int tf32) {
   return 3 * pl.accw + acts <= kTcsTmemCols ? 1 : 0;
 }
 
-void mlp_tcs_prepare(size_t smem, int np, int tf32, int cps) {
-  const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if (tf32) cudaFuncSetAttribute(k_mlp_tcs<3, OpTf32, 1>, at, (int)smem);
-  else if (np == 3) cudaFuncSetAttribute(k_mlp_tcs<3, OpBf16, 1>, at, (int)smem);
-  else if (cps == 2) cudaFuncSetAttribute(k_mlp_tcs<1, OpBf16, 2>, at, (int)smem);
-  else cudaFuncSetAttribute(k_mlp_tcs<1, OpBf16, 1>, at, (int)smem);
+void mlp_tcs_prepare(int np, int tf32, int cps) {
+  if (tf32) allow_dynamic_smem(k_mlp_tcs<3, OpTf32, 1>);
+  else if (np == 3) allow_dynamic_smem(k_mlp_tcs<3, OpBf16, 1>);
+  else if (cps == 2) allow_dynamic_smem(k_mlp_tcs<1, OpBf16, 2>);
+  else allow_dynamic_smem(k_mlp_tcs<1, OpBf16, 1>);
 }
 
 size_t mlp_tcp_smem(int nl, const int *sizes, int resnet, int np, bool dz_bf16) {
@@ -1268,23 +1267,20 @@ size_t mlp_tc_smem(int nl, int maxh, int resnet, bool dz_bf16, int np) {
   return b;
 }
 
-void mlp_tc_prepare(size_t smem, bool dz_bf16, int np) {
-  const int s = (int)smem;
-  const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+void mlp_tc_prepare(bool dz_bf16, int np) {
   if (np == 3) {
-    if (dz_bf16) cudaFuncSetAttribute(k_mlp_tc<__nv_bfloat16, 3>, at, s);
-    else cudaFuncSetAttribute(k_mlp_tc<float, 3>, at, s);
+    if (dz_bf16) allow_dynamic_smem(k_mlp_tc<__nv_bfloat16, 3>);
+    else allow_dynamic_smem(k_mlp_tc<float, 3>);
   } else {
-    if (dz_bf16) cudaFuncSetAttribute(k_mlp_tc<__nv_bfloat16, 1>, at, s);
-    else cudaFuncSetAttribute(k_mlp_tc<float, 1>, at, s);
+    if (dz_bf16) allow_dynamic_smem(k_mlp_tc<__nv_bfloat16, 1>);
+    else allow_dynamic_smem(k_mlp_tc<float, 1>);
   }
 }
 
-void mlp_tcp_prepare(size_t smem, int np, bool dz_bf16) {
-  const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if (np == 3) cudaFuncSetAttribute(k_mlp_tcp<3, float>, at, (int)smem);
-  else if (dz_bf16) cudaFuncSetAttribute(k_mlp_tcp<1, __nv_bfloat16>, at, (int)smem);
-  else cudaFuncSetAttribute(k_mlp_tcp<1, float>, at, (int)smem);
+void mlp_tcp_prepare(int np, bool dz_bf16) {
+  if (np == 3) allow_dynamic_smem(k_mlp_tcp<3, float>);
+  else if (dz_bf16) allow_dynamic_smem(k_mlp_tcp<1, __nv_bfloat16>);
+  else allow_dynamic_smem(k_mlp_tcp<1, float>);
 }
 
 void launch_mlp_tc(const MlpTcArgs &a, cudaStream_t st, long &launches) {

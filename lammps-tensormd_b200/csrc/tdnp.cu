@@ -171,15 +171,12 @@ size_t tdnp_warp_floats(const int nl[3], int maxw) {
   return (size_t)maxw * ((2 * nl[0] + 1) + 2 * nl[1] + 2 * nl[2] + 4);
 }
 
+void mlp_tdnp_prepare() { allow_dynamic_smem(k_mlp_tdnp); }
+
 int launch_mlp_tdnp(const TdnpArgs &a, cudaStream_t st, long &launches) {
   if (a.n <= 0) return 0;
   const size_t smem = a.warp_floats * sizeof(float) * kTdnpWarps;
   if (smem > 227 * 1024) return -1;
-  static size_t prepared = 0;
-  if (smem > 48 * 1024 && smem > prepared) {
-    cudaFuncSetAttribute(k_mlp_tdnp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    prepared = smem;
-  }
   int grid = (a.n + kTdnpWarps - 1) / kTdnpWarps;
   if (grid > 148 * 16) grid = 148 * 16;
   k_mlp_tdnp<<<grid, 32 * kTdnpWarps, smem, st>>>(a);

@@ -103,6 +103,23 @@ struct DescArgs {
 };
 void launch_descriptor(const DescArgs &a, cudaStream_t st, long &launches);
 
+// Dynamic shared memory of a kernel up to what the current device allows.  The
+// attribute belongs to the kernel, not to a model: set to one net's own size it
+// would take the larger launches of another model away.
+template <class Kernel>
+cudaError_t allow_dynamic_smem(Kernel *kern) {
+  cudaFuncAttributes fa{};
+  int dev = 0, optin = 0;
+  cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             optin - (int)fa.sharedSizeBytes);
+  return e;
+}
+
 // MLP forward + backward over element-grouped tiles.
 struct MlpLayer {
   int K, N;
@@ -218,13 +235,14 @@ struct TdnpArgs {
 };
 size_t tdnp_warp_floats(const int nl[3], int maxw);
 // 0, or -1 when the nets need more shared memory than a CTA has.
+void mlp_tdnp_prepare();
 int launch_mlp_tdnp(const TdnpArgs &a, cudaStream_t st, long &launches);
 size_t mlp_tc_smem(int nl, int maxh, int resnet, bool dz_bf16, int np);
-void mlp_tc_prepare(size_t smem, bool dz_bf16, int np);
+void mlp_tc_prepare(bool dz_bf16, int np);
 // Persistent form: dynamic shared memory for sizes[0..nl], 0 if unsupported
 // (residual layers).
 size_t mlp_tcp_smem(int nl, const int *sizes, int resnet, int np, bool dz_bf16);
-void mlp_tcp_prepare(size_t smem, int np, bool dz_bf16);
+void mlp_tcp_prepare(int np, bool dz_bf16);
 // Streamed-weight persistent form (weights too large to stay in shared
 // memory): dynamic shared memory and weight stages, 0 if unsupported
 // (residual layers, widths not multiples of the chunk (64 BF16 / 32 TF32
@@ -232,7 +250,7 @@ void mlp_tcp_prepare(size_t smem, int np, bool dz_bf16);
 // 3xTF32 operand format.
 size_t mlp_tcs_smem(int nl, const int *sizes, int resnet, int np, int tf32, int cps,
                     int *stages);
-void mlp_tcs_prepare(size_t smem, int np, int tf32, int cps);
+void mlp_tcs_prepare(int np, int tf32, int cps);
 // 3xTF32: 1 when TMEM holds a second hi accumulator (MlpTcArgs::hi2).
 int mlp_tcs_hi2(int nl, const int *sizes, int np, int tf32);
 
@@ -250,7 +268,7 @@ float tf32_round_host(float v);
 // weights e4m3(W * wscale) in 8x16 core matrices, per-row operand scales.
 void launch_mlp_fp8(const MlpTcArgs &a, cudaStream_t st, long &launches);
 size_t mlp_fp8_smem(int nl, int maxh, int resnet, bool dz_bf16);
-void mlp_fp8_prepare(size_t smem, bool dz_bf16);
+void mlp_fp8_prepare(bool dz_bf16);
 void pack_core_chunks_fp8(const float *src, int rows, int cols, long ld_r, long ld_k,
                           float scale, uint8_t *dst);
 
