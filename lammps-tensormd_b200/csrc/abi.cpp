@@ -460,7 +460,18 @@ int map_types(const tmd_model *m, int n, const int *type, std::vector<int> &elem
   return TMD_OK;
 }
 
-int mlp_tiles(tmd_system *s, const int *cnt, std::vector<int> &tiles) {
+size_t mlp_scratch_f4(const tmd_model *m, size_t natoms) {
+  size_t most = 0;
+  if (m->mlp_tr > 0) return most;
+  for (const MlpPlan::Form &f : m->mlp.form) {
+    if (f.ctas == 0) continue;
+    const size_t tiles = std::min(natoms / f.rows + m->h.nelt, (size_t)m->mlp.nsm * f.ctas);
+    most = std::max(most, tiles * f.scratch_f4);
+  }
+  return most;
+}
+
+void mlp_tiles(tmd_system *s, const int *cnt, std::vector<int> &tiles) {
   const tmd_model *m = s->m;
   const int nelt = m->h.nelt;
   int rows = m->mlp_tr;
@@ -476,19 +487,6 @@ int mlp_tiles(tmd_system *s, const int *cnt, std::vector<int> &tiles) {
       tiles.push_back(std::min(rows, cnt[e] - o));
     }
   s->ntiles = (int)tiles.size() / 3;
-  if (m->mlp_tr == 0) {
-    const MlpPlan::Form &f = m->mlp.form[s->mlp_form];
-    const size_t need = (size_t)std::min(s->ntiles, m->mlp.nsm * f.ctas) * f.scratch_f4;
-    if (need > s->mlp_scratch_alloc) {
-      TMD_CUDA(cudaStreamSynchronize(s->st));
-      drop_graph(s);  // captured steps hold the old scratch
-      dfree(s->mlp_scratch);
-      s->mlp_scratch_alloc = 0;
-      TMD_CUDA(dalloc(&s->mlp_scratch, need));
-      s->mlp_scratch_alloc = need;
-    }
-  }
-  return TMD_OK;
 }
 
 int set_elements(tmd_system *s, int n, const int *elem) {
@@ -506,8 +504,7 @@ int set_elements(tmd_system *s, int n, const int *elem) {
   std::vector<int> perm(n > 0 ? n : 1), fill(start.begin(), start.end() - 1);
   for (int i = 0; i < ne; i++) perm[fill[elem[i]]++] = i;
   std::vector<int> tiles;
-  const int rc = mlp_tiles(s, cnt.data(), tiles);
-  if (rc) return rc;
+  mlp_tiles(s, cnt.data(), tiles);
   if (n > 0) {
     TMD_CUDA(cudaMemcpyAsync(s->elem, s->h_elem.data(), n * sizeof(int), cudaMemcpyHostToDevice,
                              s->st));
@@ -1250,6 +1247,7 @@ int tmd_system_create(const tmd_model *m, int natoms_cap, double skin,
   A(partial, 1024 * 8); A(scal, 10);
   A(flag, 2); A(status, 2);  // flag[0] rebuild pending, flag[1] rebuilds done
   A(perm, N); A(tiles, 3 * (N / (m->mlp_tr > 0 ? m->mlp_tr : m->mlp.form[0].rows) + h.nelt + 1));
+  if (m->mlp_tr == 0) A(mlp_scratch, mlp_scratch_f4(m, N));
 #undef A
   if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void **>(&s->h_scal), 10 * sizeof(double));
   if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void **>(&s->h_status), 4 * sizeof(int));
@@ -1333,6 +1331,7 @@ int tmd_system_set_atoms(tmd_system *s, int n, const double *x, const int *type,
   std::vector<int> elem;
   int rc = map_types(s->m, n, type, elem);
   if (rc) return rc;
+  s->have_atoms = false;  // until every array holds the new ones
   s->nghost = 0;
   rc = set_elements(s, n, elem.data());
   if (rc) return rc;
@@ -1389,6 +1388,7 @@ int tmd_system_set_atoms_ghost(tmd_system *s, int nlocal, int nghost, const doub
   std::vector<int> elem;
   rc = map_types(s->m, n, type, elem);
   if (rc) return rc;
+  s->have_atoms = false;  // until every array holds the new ones
   s->nghost = nghost;
   rc = set_elements(s, n, elem.data());
   if (rc) return rc;

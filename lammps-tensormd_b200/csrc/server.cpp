@@ -138,17 +138,11 @@ size_t server_bytes_per_atom(const tmd_model *m, int cap) {
   return a;
 }
 
-// Device bytes of the FP32 MLP's tile list and act' scratch for up to `atoms`
-// atoms: the scratch grows with the tiles until every CTA slot has its own.
+// Device bytes of the FP32 MLP's tile list and act' scratch for up to `atoms` atoms.
 size_t server_mlp_bytes(const tmd_model *m, size_t atoms) {
   if (m->mlp_tr > 0) return 0;
-  size_t most = 0;
-  for (const MlpPlan::Form &f : m->mlp.form) {
-    if (f.ctas == 0) continue;
-    const size_t tiles = std::min(atoms / f.rows + m->h.nelt, (size_t)m->mlp.nsm * f.ctas);
-    most = std::max(most, tiles * f.scratch_f4 * sizeof(float4));
-  }
-  return most + 12 * (atoms / m->mlp.form[0].rows + m->h.nelt + 1);
+  return mlp_scratch_f4(m, atoms) * sizeof(float4) +
+         12 * (atoms / m->mlp.form[0].rows + m->h.nelt + 1);
 }
 
 // Row length (a multiple of 32) a job of n atoms in box volume vol needs.
@@ -286,8 +280,7 @@ int relayout(tmd_server *sv, const std::vector<JobP> &next) {
   // cell by cell
   std::vector<int> cur(B, 0), estart((size_t)C * B), tiles;
   for (int e = 1; e < B; e++) cur[e] = cur[e - 1] + total[e - 1];
-  int rc = mlp_tiles(s, total.data(), tiles);
-  if (rc) return rc;
+  mlp_tiles(s, total.data(), tiles);
   for (int c = 0; c < C; c++)
     for (int e = 0; e < B; e++) {
       estart[(size_t)c * B + e] = cur[e];
@@ -296,7 +289,7 @@ int relayout(tmd_server *sv, const std::vector<JobP> &next) {
   s->ncells = C;
   s->h_coff = coff;
   s->h_acell.clear();
-  rc = cells_geometry(s, boxes.data(), pbc.data());
+  int rc = cells_geometry(s, boxes.data(), pbc.data());
   if (rc) return rc;
   TMD_CUDA(cudaMemcpyAsync(s->coff, coff.data(), (C + 1) * sizeof(int), cudaMemcpyHostToDevice,
                            s->st));

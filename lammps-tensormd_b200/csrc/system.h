@@ -92,8 +92,7 @@ struct tmd_system {
   int *perm = nullptr, *tiles = nullptr;
   int ntiles = 0;
   int mlp_form = 0;                 // FP32 MLP form of the current tiles
-  float4 *mlp_scratch = nullptr;    // its act' scratch
-  size_t mlp_scratch_alloc = 0;
+  float4 *mlp_scratch = nullptr;    // act' scratch of every form, for natoms_cap atoms
   double *thermo_d = nullptr;
   long thermo_alloc = 0;
   // host
@@ -195,9 +194,12 @@ int map_types(const tmd_model *m, int n, const int *type, std::vector<int> &elem
 // Set n atoms' elements: host mirror, device elem[], MLP element grouping
 // (perm, tiles).  Synchronises the stream.
 int set_elements(tmd_system *s, int n, const int *elem);
+// act' scratch of the FP32 MLP in float4: the most that any form takes for up
+// to natoms atoms (it grows with the tiles until every CTA slot has its own).
+size_t mlp_scratch_f4(const tmd_model *m, size_t natoms);
 // MLP tiles (element, start, count) of atoms grouped by element, cnt[e] of
-// element e; sets ntiles, and the FP32 form and its scratch.
-int mlp_tiles(tmd_system *s, const int *cnt, std::vector<int> &tiles);
+// element e; sets ntiles and the FP32 form.
+void mlp_tiles(tmd_system *s, const int *cnt, std::vector<int> &tiles);
 // Multi-cell mode (batch.cpp): device arrays for up to max_cells cells, the
 // cell layout (atoms per cell, concatenated), per-cell boxes.
 int cells_alloc(tmd_system *s, int max_cells);
