@@ -208,6 +208,17 @@ int tmd_system_set_variant(tmd_system *sys, int family, int variant);
 int tmd_system_get_variant(tmd_system *sys, int family, int *variant);
 int tmd_system_autotune(tmd_system *sys, int family, int reps, double *ms);
 
+/* Tile height of the FP32 MLP.  The library picks one of four heights (atoms
+ * per tile) by the atoms per element; sums do not depend on it, so results are
+ * the same bit for bit.  set_mlp_rows fixes one from the next set_atoms on (0:
+ * the library's choice again), for tests and timing; TMD_ERR_ARG if the
+ * potential's MLP has no form of that height.  mlp_rows returns the height in
+ * use (0 before set_atoms) and, in forms[4], the heights there are (0 where
+ * one does not fit).  TMD_ERR_STATE for potentials in other precisions and
+ * temperature-dependent ones. */
+int tmd_system_set_mlp_rows(tmd_system *sys, int rows);
+int tmd_system_mlp_rows(tmd_system *sys, int *rows, int forms[4]);
+
 /* CUDA stream of the system (cudaStream_t as void*), for event timing. */
 int tmd_system_stream(tmd_system *sys, void **stream);
 

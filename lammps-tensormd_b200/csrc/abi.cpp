@@ -476,7 +476,7 @@ void mlp_tiles(tmd_system *s, const int *cnt, std::vector<int> &tiles) {
   const int nelt = m->h.nelt;
   int rows = m->mlp_tr;
   if (rows == 0) {
-    s->mlp_form = mlp_fp32_form(m->mlp, cnt, nelt);
+    s->mlp_form = s->mlp_force >= 0 ? s->mlp_force : mlp_fp32_form(m->mlp, cnt, nelt);
     rows = m->mlp.form[s->mlp_form].rows;
   }
   tiles.clear();
@@ -1707,6 +1707,30 @@ int tmd_system_autotune(tmd_system *s, int family, int reps, double *ms) {
   if (rc) return rc;
   // results of the chosen form (the forms round differently)
   return tmd_compute(s, 0, 0, 1.0, nullptr, nullptr, nullptr, nullptr, nullptr);
+}
+
+int tmd_system_set_mlp_rows(tmd_system *s, int rows) {
+  if (!s || rows < 0) return fail(TMD_ERR_ARG, "bad tile height");
+  if (s->m->mlp_tr > 0) return fail(TMD_ERR_STATE, "not an FP32 MLP");
+  if (rows == 0) {
+    s->mlp_force = -1;
+    return TMD_OK;
+  }
+  for (int v = 0; v < 4; v++)
+    if (s->m->mlp.form[v].ctas > 0 && s->m->mlp.form[v].rows == rows) {
+      s->mlp_force = v;
+      return TMD_OK;
+    }
+  return fail(TMD_ERR_ARG, "no MLP form has tiles of " + std::to_string(rows) + " atoms");
+}
+
+int tmd_system_mlp_rows(tmd_system *s, int *rows, int forms[4]) {
+  if (!s) return fail(TMD_ERR_ARG, "null system");
+  if (s->m->mlp_tr > 0) return fail(TMD_ERR_STATE, "not an FP32 MLP");
+  if (rows) *rows = s->have_atoms ? s->m->mlp.form[s->mlp_form].rows : 0;
+  for (int v = 0; forms && v < 4; v++)
+    forms[v] = s->m->mlp.form[v].ctas > 0 ? s->m->mlp.form[v].rows : 0;
+  return TMD_OK;
 }
 
 int tmd_system_stream(tmd_system *s, void **stream) {

@@ -92,6 +92,7 @@ struct tmd_system {
   int *perm = nullptr, *tiles = nullptr;
   int ntiles = 0;
   int mlp_form = 0;                 // FP32 MLP form of the current tiles
+  int mlp_force = -1;               // the caller's choice, -1: the library's
   float4 *mlp_scratch = nullptr;    // act' scratch of every form, for natoms_cap atoms
   double *thermo_d = nullptr;
   long thermo_alloc = 0;

@@ -42,6 +42,8 @@ SIGNATURES = [
     ("tmd_system_set_variant", _c_int, [_vp, _c_int, _c_int]),
     ("tmd_system_get_variant", _c_int, [_vp, _c_int, _pi]),
     ("tmd_system_autotune", _c_int, [_vp, _c_int, _c_int, _pd]),
+    ("tmd_system_set_mlp_rows", _c_int, [_vp, _c_int]),
+    ("tmd_system_mlp_rows", _c_int, [_vp, _pi, _pi]),
     ("tmd_system_stream", _c_int, [_vp, ctypes.POINTER(_vp)]),
     ("tmd_system_launches", _c_long, [_vp]),
     ("tmd_system_rebuilds", _c_int, [_vp, _pl]),

@@ -202,6 +202,16 @@ class TensorMDSystem:
         check(self.lib.tmd_system_get_variant(self.h, 1, ctypes.byref(v)))
         return self.DESC_VARIANTS[v.value]
 
+    # tile height of the FP32 MLP
+    def set_mlp_rows(self, rows: int):
+        check(self.lib.tmd_system_set_mlp_rows(self.h, int(rows)))
+
+    def mlp_rows(self):
+        """(atoms per tile in use, the heights there are)."""
+        r, forms = ctypes.c_int(), np.zeros(4, dtype=np.int32)
+        check(self.lib.tmd_system_mlp_rows(self.h, ctypes.byref(r), _ip(forms)))
+        return r.value, [int(f) for f in forms]
+
     def autotune(self, reps: int = 5, family: str = "force"):
         """Time every form of a kernel family ("force" or "descriptor") on the
         current atoms, keep the fastest; returns {form: ms per launch}."""

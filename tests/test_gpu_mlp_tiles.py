@@ -3,10 +3,12 @@
 The tile height follows the number of atoms (1, 2, 4 or 8 rows per thread) and
 the block width the widest hidden layer (32, 64, 128 columns; wider layers take
 several blocks).  Sums run over the reduction index in one order whatever the
-tile, so a cell's results must not depend on how many cells share the launch:
-one cell (smallest tiles) against the oracle, then the same cell among enough
-copies to reach the larger tiles, bitwise.  Cell sizes put every element's last
-tile at one row, a full tile and one row more."""
+tile, so a cell's results must not depend on the tile height or on how many
+cells share the launch.  test_tiles_and_blocks: one cell (smallest tiles) against
+the oracle, then the same cell among copies of it, bitwise, with the heights that
+the library picks.  test_every_tile_height: every height of every block width,
+bitwise against the smallest and that against the oracle, with one element's
+atoms at one row less than a tile, a full tile and one row more."""
 import numpy as np
 import pytest
 
@@ -54,3 +56,40 @@ def test_tiles_and_blocks(tmp_path, net):
             assert np.array_equal(many["f"].reshape(copies, -1, 3),
                                   np.broadcast_to(out["f"], (copies,) + out["f"].shape))
             b.close()
+
+
+WIDTHS = [dict(hidden=(24, 32), actfn=1),
+          dict(hidden=(64, 64, 64), actfn=2, resnet=1),
+          dict(hidden=(128, 100), actfn=3)]
+
+
+@pytest.mark.parametrize("net", WIDTHS, ids=["32", "64", "128"])
+def test_every_tile_height(tmp_path, net):
+    p = tmp_path / "m.npz"
+    syms = synth.gaussian_potential(p, nelt=2, num_filters=4, rc=4.5, max_moment=2, seed=3, **net)
+    m = TensorMDModel(f"{p} {' '.join(syms)}")
+    orc = Oracle(load_npz(p))
+    rng = np.random.default_rng(4)
+    x, box = synth.lattice("fcc", 3.6, 5, 4, 4)
+    x = synth.wrap(x + rng.normal(0.0, 0.08, x.shape), box)
+    s = TensorMDSystem(m, len(x), 1.0)
+    s.set_box(box)
+    heights = s.mlp_rows()[1]
+    block = 32 if max(net["hidden"]) <= 32 else (64 if max(net["hidden"]) <= 64 else 128)
+    assert heights == [1024 // block * r for r in (1, 2, 4, 8)]
+    for first in sorted({h + d for h in heights for d in (-1, 0, 1)}):
+        t = np.full(len(x), 2, dtype=np.int32)
+        t[:first] = 1
+        got = []
+        for h in heights:
+            s.set_mlp_rows(h)
+            s.set_atoms(x, t)
+            assert s.mlp_rows()[0] == h
+            got.append(s.compute(1, 1))
+        ref = orc.compute(x, t - 1, box, [1, 1, 1], skin=1.0)
+        assert rel_rms(got[0]["f"], ref["f"]) <= 1e-5
+        for g in got[1:]:
+            assert np.array_equal(g["f"], got[0]["f"]) and g["energy"] == got[0]["energy"]
+    s.set_mlp_rows(0)
+    s.set_atoms(x, t)
+    assert s.mlp_rows()[0] in heights
