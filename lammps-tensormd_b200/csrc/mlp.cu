@@ -1,6 +1,7 @@
 // mlp.cu -- FP32 MLP: shape limits, forms, weight packing and dispatch
 // (kernel and semantics in mlp_impl.cuh).
 #include <algorithm>
+#include <cmath>
 #include <string>
 #include <vector>
 
@@ -75,16 +76,28 @@ MlpPlan mlp_fp32_plan(int nl, const int *sizes, int actfn, int resnet, int nsm) 
 }
 
 int mlp_fp32_form(const MlpPlan &p, const int *count, int nelt) {
-  // Time of the busiest SM in microseconds for 64-wide hidden layers (other
-  // widths scale all four alike), from timings on the B200: a tile alone on an
-  // SM takes lat (bound by latency), tiles that share an SM thr each (bound by
-  // shared memory for 1 and 2 row registers, by the FMA pipe for 4 and 8).
-  // Large tiles win once every SM has some; below that, small ones spread the
-  // atoms over more SMs.  Measured with 1 / 2 / 4 / 8 row registers: 4,000
-  // atoms 15.7 / 12.7 / 23 / 32 us, 23,040 atoms of a 128-wide net - / 231 /
-  // 151 / 143, 128,000 atoms - / 196 / 145 / 155, 1,048,576 atoms - / 2087 /
-  // 1673 / 1506.
-  static const double lat[4] = {10.0, 13.6, 25.0, 37.0}, thr[4] = {7.0, 7.4, 10.0, 19.4};
+  // Time of the busiest SM, in units of one tile of 4 row registers on an SM
+  // full of them, from timings of all forms inside a step on the B200 (five
+  // nets of the three block widths, 108 to 400,000 atoms).  With every CTA slot
+  // taken a tile costs thr (1 and 2 row registers are bound by shared memory, 4
+  // and 8 by the FMA pipe).  The last, partial wave takes lat for its first
+  // tile on an SM (bound by latency) and 0.75 thr for each further one beside
+  // it.  In a grid of several waves the first 148 CTAs do not lie on 148 SMs:
+  // from about 108 tiles (0.73 of the SMs) on, the last wave has two on one SM
+  // (128,000 atoms in 1,000 tiles 162 us, 126,976 in 992 tiles 140).  Small
+  // tiles spread few atoms over more SMs, large ones read the weights less
+  // often: 8 row registers lose at 32 columns, where a tile has too few
+  // weights to fill the pipe, and win at 64 and 128 once their waves are
+  // nearly full.
+  // Over that sweep the choice is within 0.2 / 0.2 / 0.6% of the best form on
+  // average at 32 / 64 / 128 columns, within 3 / 6 / 9% at worst (one table for
+  // all widths: 7.6 / 1.1 / 2.2%, 50 / 14 / 14%).  Times with 1 / 2 / 4 / 8 row
+  // registers: 64-64-64 net, 4,000 atoms 19.6 / 18.7 / 27.5 / 37.4 us, 128,000
+  // atoms - / 202 / 150 / 162; 32-wide net, 97,556 atoms 140 / 112 / 107 / 150;
+  // 128-128x3 net, 23,328 atoms 316 / 235 / 155 / 146.
+  static const double kLat[3][4] = {{0.84, 1.17, 2.22, 3.18}, {1.16, 1.20, 2.10, 3.04}, {0.97, 1.34, 1.71, 2.57}};
+  static const double kThr[3][4] = {{0.41, 0.57, 1.0, 3.08}, {0.48, 0.66, 1.0, 1.77}, {0.57, 0.81, 1.0, 1.64}};
+  const int w = p.nt == 32 ? 0 : (p.nt == 64 ? 1 : 2);
   int best = -1;
   double best_c = 0.0;
   for (int v = 0; v < 4; v++) {
@@ -92,10 +105,12 @@ int mlp_fp32_form(const MlpPlan &p, const int *count, int nelt) {
     if (ctas == 0) continue;
     long tiles = 0;
     for (int e = 0; e < nelt; e++) tiles += mlp_cdiv(count[e], p.form[v].rows);
-    const long slots = (long)p.nsm * ctas;
-    const long t = tiles <= slots ? (tiles + p.nsm - 1) / p.nsm
-                                  : (tiles + slots - 1) / slots * ctas;
-    const double c = std::max(lat[v], t * thr[v]);
+    const long waves = tiles / ((long)p.nsm * ctas), rest = tiles - waves * p.nsm * ctas;
+    double c = (double)waves * ctas * kThr[w][v];
+    if (rest > 0) {  // with `deep` tiles of the last wave on the busiest SM
+      const double deep = std::ceil((double)rest / p.nsm + (waves > 0 ? 0.27 : 0.0));
+      c += kLat[w][v] + 0.75 * (std::min(deep, (double)ctas) - 1.0) * kThr[w][v];
+    }
     if (best < 0 || c < best_c) { best = v; best_c = c; }
   }
   return best;

@@ -93,3 +93,27 @@ def test_every_tile_height(tmp_path, net):
     s.set_mlp_rows(0)
     s.set_atoms(x, t)
     assert s.mlp_rows()[0] in heights
+
+
+# (hidden layers, atoms): the heights that the choice must be among, each at
+# least 5% faster than the others in timings of all four (1,024 / block width x
+# 1, 2, 4, 8 atoms; the 128,000 and 126,976 atoms differ in how full the last
+# wave of 128-atom tiles is)
+CHOICES = [((32, 32, 32), 432, (32,)), ((32, 32, 32), 97556, (64, 128)),
+           ((64, 64), 432, (16,)), ((64, 64), 8192, (32,)), ((64, 64), 126976, (128,)),
+           ((64, 64), 128000, (64,)),
+           ((128, 128, 128), 432, (8,)), ((128, 128, 128), 2048, (16,)),
+           ((128, 128, 128), 23040, (64,)), ((128, 128, 128), 202612, (32, 64))]
+
+
+@pytest.mark.parametrize("hidden,n,best", CHOICES, ids=[f"{h[0]}-{n}" for h, n, _ in CHOICES])
+def test_height_follows_the_timings(tmp_path, hidden, n, best):
+    p = tmp_path / "m.npz"
+    syms = synth.gaussian_potential(p, nelt=1, num_filters=4, rc=2.0, max_moment=1, seed=3,
+                                    hidden=hidden, actfn=2)
+    s = TensorMDSystem(TensorMDModel(f"{p} {' '.join(syms)}"), n, 0.5)
+    k = int(np.ceil(n ** (1 / 3)))
+    s.set_box(np.array([0, 0, 0, 3.0 * k, 3.0 * k, 3.0 * k, 0, 0, 0]))
+    x = 3.0 * np.stack(np.unravel_index(np.arange(n), (k, k, k)), -1).astype(float)
+    s.set_atoms(x, np.ones(n, dtype=np.int32))
+    assert s.mlp_rows()[0] in best
