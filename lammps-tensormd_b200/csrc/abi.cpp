@@ -352,14 +352,15 @@ DescArgs desc_args(tmd_system *s, int variant) {
 }
 
 // The descriptor form in use: the caller's or the autotuner's choice, else the
-// wide form, and for table radials on many atoms the split one (measured on
-// the B200, k_pair_geo + k_descriptor_c against k_descriptor_w: 23,040 atoms
-// of a 32-filter table potential 162 against 187 us; at 430 atoms the second
-// launch costs more than it gives, and the Gaussian kinds gain under 3%).
+// wide form, and for table radials on many atoms the split one (inside a step
+// on the B200, wide against split: 32 filters, 23,276 atoms 189 against 180 us,
+// 12,312 atoms 111 / 100, 8,192 atoms 82 / 87, 1,458 atoms 32 / 43; 64 filters
+// 353 / 308, 200 / 177, 147 / 131, 50 / 48; the Gaussian kinds gain under 3%).
+// Back to back, with the neighbours' positions still in L2, the two are equal.
 // Both sum the pairs in the same order: the results are the same bit for bit.
 int desc_form(const tmd_system *s) {
   if (s->desc_variant >= 0) return s->desc_variant;
-  return s->m->kp.radial == 1 && s->n >= 8192 ? kDescSplit : kDescWide;
+  return s->m->kp.radial == 1 && s->n - s->nghost >= 8192 ? kDescSplit : kDescWide;
 }
 
 int default_force_variant(const tmd_model *m) {

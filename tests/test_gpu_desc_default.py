@@ -1,12 +1,12 @@
-"""Default descriptor form: wide, and split for table radials on 8,192 atoms
-and more.  The choice follows the atom count of the launch, so a cell must get
+"""Default descriptor form: wide, and split for table radials on 8,192 (local)
+atoms and more.  The choice follows the atom count of the launch, so a cell must get
 the same bits from both forms: descriptors, forces, energy and virial of the
 wide and the split form are compared bitwise over filter counts, radial kinds,
 ranks and elements."""
 import numpy as np
 import pytest
 
-from tmd_b200 import TensorMDModel, TensorMDSystem, synth
+from tmd_b200 import TensorMDBatch, TensorMDModel, TensorMDSystem, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -46,3 +46,45 @@ def test_default_follows_kind_and_size(tmp_path):
     assert s.descriptor_variant() == "split"
     s.set_descriptor_variant("wide")  # the caller's choice stands
     assert s.descriptor_variant() == "wide"
+
+
+def test_default_counts_local_atoms(tmp_path):
+    p = tmp_path / "m.npz"
+    syms = synth.gaussian_potential(p, rc=3.0, hidden=(16,), actfn=2, seed=8, nelt=1,
+                                    num_filters=8, max_moment=1)
+    m = TensorMDModel(f"{p} {' '.join(syms)} interp 0.005")
+    x, _, _, _ = synth.build_system("bcc", 2.9, (16, 16, 17), sigma=0.05, nelt=1, seed=6)
+    t = np.ones(len(x), dtype=np.int32)
+    s = TensorMDSystem(m, len(x), 0.5)
+    s.set_atoms_ghost(8191, x, t)  # the kernels run over the local atoms
+    assert s.descriptor_variant() == "wide"
+    s.set_atoms_ghost(8192, x, t)
+    assert s.descriptor_variant() == "split"
+
+
+@pytest.mark.parametrize("nelt,K", [(1, 16), (3, 32)])
+def test_wide_and_split_agree_bitwise_in_batches(tmp_path, nelt, K):
+    """Cells of one batch, each with its own box, above the split form's line."""
+    p = tmp_path / "m.npz"
+    syms = synth.gaussian_potential(p, rc=5.0, hidden=(16, 16), actfn=2, seed=8, nelt=nelt,
+                                    num_filters=K, max_moment=3)
+    m = TensorMDModel(f"{p} {' '.join(syms)} interp 0.005")
+    cells = [synth.build_system(lat, a, rep, sigma=0.08, nelt=nelt, seed=k)[:3]
+             for k in range(24) for lat, a, rep in (("bcc", 2.9, (5, 5, 6)), ("fcc", 3.6, (3, 4, 3)))]
+    b = TensorMDBatch(m, [len(c[0]) for c in cells], 1.0)
+    b.set_cells(np.stack([c[2] for c in cells]))
+    b.set_atoms(np.concatenate([c[0] for c in cells]), np.concatenate([c[1] for c in cells]))
+    assert sum(len(c[0]) for c in cells) >= 8192
+    assert b.system().descriptor_variant() == "split"
+    got = {}
+    for form in ("split", "wide"):
+        b.system().set_descriptor_variant(form)
+        got[form] = b.compute()
+    for k in got["split"]:
+        assert np.array_equal(got["split"][k], got["wide"][k]), k
+    k = int(np.argmax([len(c[0]) for c in cells]))  # a cell alone gives the same forces
+    s = TensorMDSystem(m, len(cells[k][0]), 1.0)
+    s.set_box(cells[k][2])
+    s.set_atoms(cells[k][0], cells[k][1])
+    at = sum(len(c[0]) for c in cells[:k])
+    assert np.array_equal(s.compute(1, 1)["f"], got["split"]["f"][at:at + len(cells[k][0])])
