@@ -246,8 +246,12 @@ int tmd_system_tdnp_energies(tmd_system *sys, double *entropy, double *free_ener
  * of their mbarriers, before any MMA or copy is issued; nothing arrives on
  * it, so each CTA takes its timeout path (no asynchronous work in flight,
  * TMEM freed) and tmd_compute returns TMD_ERR_TIMEOUT with the context still
- * usable.  cycles = 0 (the default) turns it off; the FP32 MLP's bounded
- * waits (copies of its weight stream) are not probed. */
+ * usable.  In the FP32 MLP one side of every CTA leaves at once and the
+ * other's waits take `cycles` as their limit: the producer for an even number
+ * (the consumers wait for a chunk that never comes), the consumers for an odd
+ * one (the producer fills its ring, waits for a stage that nobody releases,
+ * and drains its copies; nets of more chunks than stages, which all but the
+ * smallest are).  cycles = 0 (the default) turns it off. */
 int tmd_system_set_wait_probe(tmd_system *sys, long long cycles);
 
 /* Measured FP32 issue peak of a device: a packed-FMA (FFMA2) kernel with

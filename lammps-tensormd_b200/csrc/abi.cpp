@@ -428,6 +428,8 @@ void launch_force_eval(tmd_system *s, float scale, bool want_vatom) {
     ma.nt = pl.nt; ma.form = s->mlp_form; ma.nchunk = pl.nchunk;
     ma.grid = std::min(s->ntiles, pl.nsm * f.ctas); ma.smem = f.smem;
     ma.stream = m->d_mlp_stream; ma.scratch = s->mlp_scratch; ma.scratch_f4 = f.scratch_f4;
+    ma.wait_cycles = s->wait_probe;
+    ma.probe = s->wait_probe == 0 ? 0 : (s->wait_probe % 2 ? kMlpProbeProducer : kMlpProbeConsumer);
     ma.status = s->status; ma.ntiles = s->ntiles; ma.tiles = s->tiles; ma.perm = s->perm;
     ma.G = s->G; ma.dEdG = s->dEdG; ma.E = s->E; ma.layers = m->d_layers;
     launch_mlp_fp32(ma, s->st, s->launches);
@@ -801,7 +803,7 @@ int run_md(tmd_system *s, int nsteps, double dt, const NvtSpec *nvt, int thermo_
       row = row0;
       continue;
     }
-    if (st & kStatusTimeout) return fail(TMD_ERR_TIMEOUT, "a tensor-core wait timed out");
+    if (st & kStatusTimeout) return fail(TMD_ERR_TIMEOUT, "a bounded wait of the MLP kernel timed out");
     if (st & kStatusLaunch) return fail(TMD_ERR_CUDA, "neighbor build launched without its shared memory");
     if (st & kStatusShift) return fail(TMD_ERR_ARG, "periodic cell is too small for the cutoff");
     if (st & kStatusNonfinite) return fail(TMD_ERR_NONFINITE, "non-finite force during the run");
@@ -1494,7 +1496,7 @@ int tmd_compute(tmd_system *s, int eflag, int vflag, double scale, double *energ
     if (rc) return rc;
     return tmd_compute(s, eflag, vflag, scale, energy, virial, f, eatom, vatom);
   }
-  if (st & kStatusTimeout) return fail(TMD_ERR_TIMEOUT, "a tensor-core wait timed out");
+  if (st & kStatusTimeout) return fail(TMD_ERR_TIMEOUT, "a bounded wait of the MLP kernel timed out");
   if (st & kStatusLaunch) return fail(TMD_ERR_CUDA, "neighbor build launched without its shared memory");
   if (st & kStatusShift) return fail(TMD_ERR_ARG, "periodic cell is too small for the cutoff");
   if (st & kStatusOutside) return fail(TMD_ERR_ARG, "atom outside a non-periodic boundary");

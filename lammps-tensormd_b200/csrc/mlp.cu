@@ -135,9 +135,11 @@ void mlp_fp32_pack(int nl, const int *sizes, int nt, const std::vector<float> *W
   }
 }
 
-void launch_mlp_fp32(const MlpArgs &a, cudaStream_t st, long &launches) {
-  if (a.ntiles <= 0) return;
+void launch_mlp_fp32(const MlpArgs &args, cudaStream_t st, long &launches) {
+  if (args.ntiles <= 0) return;
   launches += 1;
+  MlpArgs a = args;
+  if (a.wait_cycles <= 0) a.wait_cycles = tc::kWaitCycles;
   switch (a.nt) {
     case 32: launch_mlp_tr<32>(a, st); break;
     case 64: launch_mlp_tr<64>(a, st); break;

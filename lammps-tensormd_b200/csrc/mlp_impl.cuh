@@ -243,12 +243,13 @@ k_mlp_fp32(MlpArgs a) {
   bool bad = false;
   auto wait = [&](uint64_t *b, uint32_t parity) {
     if (tc::mbar_test(b, parity)) return;
-    if (!tc::mbar_wait(b, parity, bad ? 1 : tc::kWaitCycles)) bad = true;
+    if (!tc::mbar_wait(b, parity, bad ? 1 : a.wait_cycles)) bad = true;
   };
   auto sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kMlpThreads) : "memory"); };
   if (w == kMlpThreads / 32) {
     // ---- producer: every chunk of this CTA's tiles into the ring, a stage
     // as soon as the four consumer warps have released it
+    if (a.probe == kMlpProbeConsumer) return;
     int st = 0, round = 0, slot = 0;
     for (int tile = blockIdx.x; tile < a.ntiles && !bad; tile += gridDim.x) {
       const int elt = __ldg(a.tiles + 3 * tile), start = __ldg(a.tiles + 3 * tile + 1),
@@ -311,6 +312,7 @@ k_mlp_fp32(MlpArgs a) {
     return;
   }
   // ---- consumer
+  if (a.probe == kMlpProbeProducer) return;
   int c_st = 0, c_g = 0;
   uint32_t c_ph = 0;
   float2 acc[TR][4];

@@ -358,7 +358,7 @@ int read_cells(tmd_server *sv) {
   if (rc) return rc;
   const int st = s->h_status[0];
   if (st & kStatusOverflow) return fail(TMD_ERR_CAPACITY, "neighbor list overflow");
-  if (st & kStatusTimeout) return fail(TMD_ERR_TIMEOUT, "a tensor-core wait timed out");
+  if (st & kStatusTimeout) return fail(TMD_ERR_TIMEOUT, "a bounded wait of the MLP kernel timed out");
   if (st & kStatusLaunch) return fail(TMD_ERR_CUDA, "neighbor build launched without its shared memory");
   if (st & kStatusShift) return fail(TMD_ERR_ARG, "a cell is too small for the cutoff");
   return TMD_OK;

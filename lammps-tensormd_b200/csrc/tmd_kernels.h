@@ -140,6 +140,10 @@ struct MlpPlan {
     size_t scratch_f4; // act' scratch per CTA (float4)
   } form[4];
 };
+// Failure-detection hook (tmd_system_set_wait_probe): one side of every CTA's
+// ring leaves at once, so the other's first wait runs out.
+constexpr int kMlpProbeConsumer = 1;  // no copies: the consumers' wait for the first chunk
+constexpr int kMlpProbeProducer = 2;  // no stage is released: the producer's, copies in flight
 struct MlpArgs {
   int nl, actfn, resnet, nin;
   int sizes[kMaxLayers + 1];
@@ -149,6 +153,8 @@ struct MlpArgs {
   float4 *scratch;      // act' of the CTAs' tiles
   size_t scratch_f4;    // per CTA
   int *status;          // timeout bit of the bounded waits
+  long long wait_cycles;  // limit of a wait, 0: the default
+  int probe;            // 0 or kMlpProbe*
   int ntiles;
   const int *tiles;   // [ntiles][3] = (element, start, count) into perm
   const int *perm;    // atom indices grouped by element

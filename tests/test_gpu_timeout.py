@@ -1,4 +1,4 @@
-"""Failure detection of the tensor-core MLP kernels, without a GPU fault.
+"""Failure detection of the MLP kernels, without a GPU fault.
 
 Every mbarrier wait in the tcgen05 kernels is bounded; a wait that runs out
 sets a status bit, the kernel drains what it issued, frees its TMEM and
@@ -8,6 +8,12 @@ arrives on, before it issues any MMA or copy: the timeout path runs with no
 asynchronous work in flight.  Each kernel form must then report the timeout,
 and the same system must compute the same results as before once the probe
 is off (the context stays usable).
+
+The FP32 kernel's waits are those of its chunk ring.  An even limit makes every
+producer warp leave (the consumers wait for a chunk that never comes), an odd
+one the consumers (the producer fills its ring, waits for a stage that nobody
+releases and drains the copies it has in flight).  Both over every tile height:
+rings of six and of three stages.
 """
 import numpy as np
 import pytest
@@ -56,3 +62,26 @@ def test_wait_timeout_is_reported_and_recovers(tmp_path, case):
     again = s.compute(1, 1)
     assert np.array_equal(again["f"], ref["f"])
     assert again["energy"] == ref["energy"]
+
+
+@pytest.mark.parametrize("cycles", [2000, 2001], ids=["no-copies", "copies-in-flight"])
+@pytest.mark.parametrize("hidden", [(32, 32), (64, 64), (128, 128, 128)], ids=["32", "64", "128"])
+def test_fp32_ring_timeout_is_reported_and_recovers(tmp_path, hidden, cycles):
+    p = tmp_path / "pot.npz"
+    syms = synth.gaussian_potential(p, seed=5, nelt=2, num_filters=16, rc=5.0, max_moment=3,
+                                    hidden=hidden, actfn=2)
+    x, t, box, _ = synth.build_system("fcc", 3.6, (6, 6, 6), sigma=0.05, nelt=2, seed=3)
+    s = TensorMDSystem(TensorMDModel(f"{p} {' '.join(syms)}"), len(x), 1.0)
+    s.set_box(box)
+    for rows in s.mlp_rows()[1]:
+        s.set_mlp_rows(rows)
+        s.set_atoms(x, t)
+        ref = s.compute(1, 1)
+        assert s.lib.tmd_system_set_wait_probe(s.h, cycles) == 0
+        with pytest.raises(TmdError) as err:
+            s.compute(1, 1)
+        assert err.value.code == TMD_ERR_TIMEOUT
+        assert s.lib.tmd_system_set_wait_probe(s.h, 0) == 0
+        again = s.compute(1, 1)
+        assert np.array_equal(again["f"], ref["f"])
+        assert again["energy"] == ref["energy"]
