@@ -313,15 +313,24 @@ __device__ inline void moments(float x, float y, float z, float M[D]) {
 // xx + yy + zz = 1 and the 20 monomials span only 16 functions on the sphere:
 // four of every five FMAs of the contractions and of the shared-memory reads
 // that feed them, and rows of 64 bytes.  The descriptor accumulates P over the
-// orthogonal set {1, x, y, z, zz - 1/3, xy, xz, xx - yy, yz, x (xx - 3/5),
-// x (yy - zz), y (yy - 3/5), y (zz - xx), z (zz - 3/5), z (xx - yy), xyz}: a
+// set {1, x, y, z, zz - c, xy, xz, xx - yy, yz, x (xx - s), x (yy - zz),
+// y (yy - s), y (zz - xx), z (zz - s), z (xx - yy), xyz}, orthogonal for c = 1/3
+// and s = 3/5: a
 // monomial's sum, put together again from orthogonal parts, carries the
 // rounding noise of its direct sum and no more (with xx - zz and the like,
 // sums over xyy came out 1.5 times as noisy).  The pair force evaluates Q(u)
 // with zz eliminated, over {1, x, y, z, xx, xy, xz, yy, yz, xxx, xxy, xxz,
 // xyy, xyz, yyy, yyz}.
+// c and s are the nearest numbers of 12 and 9 bits, so that the shares of P_0 and
+// P_x in the other sums, (1 - c) / 2 and (1 - s) / 2, are FP32 numbers too: with
+// fl(1/3) for both, xx and yy came out 4.5e-8 too large for every atom, twice
+// that in rank 2 of G: total energies of W crystals off by 8e-9 and 1.8e-8 of
+// themselves, virials by up to 2.1e-6 (1e-9, 3e-9 and 3.2e-7 with these).
 template <int D>
 constexpr int kBasis = basis_count(D);
+
+constexpr float kC2 = 1365.f / 4096.f, kC2Rest = (1.f - kC2) / 2.f;
+constexpr float kC3 = 307.f / 512.f, kC3Rest = (1.f - kC3) / 2.f;
 
 template <int D>
 __device__ inline void basis_p(float x, float y, float z, float M[kBasis<D>]) {
@@ -333,11 +342,11 @@ __device__ inline void basis_p(float x, float y, float z, float M[kBasis<D>]) {
     const float xx = __fmul_rn(x, x), yy = __fmul_rn(y, y), zz = __fmul_rn(z, z),
                 xy = __fmul_rn(x, y);
     M[0] = 1.f; M[1] = x; M[2] = y; M[3] = z;
-    M[4] = fmaf(z, z, -1.f / 3.f); M[5] = xy; M[6] = __fmul_rn(x, z);
+    M[4] = fmaf(z, z, -kC2); M[5] = xy; M[6] = __fmul_rn(x, z);
     M[7] = __fmul_rn(x - y, x + y); M[8] = __fmul_rn(y, z);
-    M[9] = __fmul_rn(x, xx - 0.6f); M[10] = __fmul_rn(x, yy - zz);
-    M[11] = __fmul_rn(y, yy - 0.6f); M[12] = __fmul_rn(y, zz - xx);
-    M[13] = __fmul_rn(z, zz - 0.6f); M[14] = __fmul_rn(z, xx - yy);
+    M[9] = __fmul_rn(x, xx - kC3); M[10] = __fmul_rn(x, yy - zz);
+    M[11] = __fmul_rn(y, yy - kC3); M[12] = __fmul_rn(y, zz - xx);
+    M[13] = __fmul_rn(z, zz - kC3); M[14] = __fmul_rn(z, xx - yy);
     M[15] = __fmul_rn(xy, z);
   }
 }
@@ -348,19 +357,18 @@ struct Rank3 {
 };
 __device__ inline Rank3 basis_expand(const float A[16]) {
   Rank3 r;
-  const float t = A[0] * (1.f / 3.f);
-  r.zz = t + A[4];
-  r.xx = fmaf(0.5f, A[7] - A[4], t);
-  r.yy = fmaf(-0.5f, A[7] + A[4], t);
-  r.xxx = fmaf(0.6f, A[1], A[9]);
-  r.xyy = fmaf(0.2f, A[1], 0.5f * (A[10] - A[9]));
-  r.xzz = fmaf(0.2f, A[1], -0.5f * (A[10] + A[9]));
-  r.yyy = fmaf(0.6f, A[2], A[11]);
-  r.yzz = fmaf(0.2f, A[2], 0.5f * (A[12] - A[11]));
-  r.xxy = fmaf(0.2f, A[2], -0.5f * (A[12] + A[11]));
-  r.zzz = fmaf(0.6f, A[3], A[13]);
-  r.xxz = fmaf(0.2f, A[3], 0.5f * (A[14] - A[13]));
-  r.yyz = fmaf(0.2f, A[3], -0.5f * (A[14] + A[13]));
+  r.zz = fmaf(kC2, A[0], A[4]);
+  r.xx = fmaf(kC2Rest, A[0], 0.5f * (A[7] - A[4]));
+  r.yy = fmaf(kC2Rest, A[0], -0.5f * (A[7] + A[4]));
+  r.xxx = fmaf(kC3, A[1], A[9]);
+  r.xyy = fmaf(kC3Rest, A[1], 0.5f * (A[10] - A[9]));
+  r.xzz = fmaf(kC3Rest, A[1], -0.5f * (A[10] + A[9]));
+  r.yyy = fmaf(kC3, A[2], A[11]);
+  r.yzz = fmaf(kC3Rest, A[2], 0.5f * (A[12] - A[11]));
+  r.xxy = fmaf(kC3Rest, A[2], -0.5f * (A[12] + A[11]));
+  r.zzz = fmaf(kC3, A[3], A[13]);
+  r.xxz = fmaf(kC3Rest, A[3], 0.5f * (A[14] - A[13]));
+  r.yyz = fmaf(kC3Rest, A[3], -0.5f * (A[14] + A[13]));
   return r;
 }
 
@@ -422,10 +430,10 @@ __device__ inline void dedp_row(const float gp[4], const float *T, int M,
     F[1] = fmaf(t11, p.xzz, t1 * A[1]);
     F[2] = fmaf(t11, p.yzz, t1 * A[2]);
     F[3] = fmaf(t10, p.zzz, t1 * A[3]);
-    F[4] = t4 * fmaf(-1.5f, A[4], 0.5f * A[7]);
+    F[4] = t4 * fmaf(kC2Rest - kC2, A[0], fmaf(-1.5f, A[4], 0.5f * A[7]));  // xx - zz
     F[5] = t5 * A[5];
     F[6] = t5 * A[6];
-    F[7] = t4 * fmaf(-1.5f, A[4], -0.5f * A[7]);
+    F[7] = t4 * fmaf(kC2Rest - kC2, A[0], fmaf(-1.5f, A[4], -0.5f * A[7]));  // yy - zz
     F[8] = t5 * A[8];
     F[9] = fmaf(t10, p.xxx, -t11 * p.xzz);
     F[10] = -t11 * A[12];
