@@ -55,6 +55,9 @@ def parse():
     ap.add_argument("--profile-precision", default="fp32",
                     choices=["fp32", "tf32x3", "bf16x3", "bf16"],
                     help="MLP precision form of the --profile-step target")
+    ap.add_argument("--profile-force", default="",
+                    choices=["", "filter_lane", "pair_lane8", "pair_lane16", "pair_lane32"],
+                    help="force form of the --profile-step target (default: the library's)")
     ap.add_argument("--profile-desc", default="", choices=["", "filter4", "wide", "wide2", "split"],
                     help="descriptor form of the --profile-step target (default: the "
                          "library's default form)")
@@ -228,8 +231,14 @@ def ncu_traffic(config, kernel):
     return None
 
 
-def algorithmic(cfg, npairs_rc, nlist, B, K, D, nin, form):
-    """Algorithmic FLOPs and HBM bytes per launch of the force kernel.
+# functions of the pair direction that the kernels sum over, by the number of
+# monomials: rank 3 takes the 16 that are independent on the unit sphere
+FUNCTIONS = {1: 1, 4: 4, 10: 10, 20: 16}
+
+
+def algorithmic(cfg, npairs_rc, nlist, B, K, D, nin, form, nfun=None):
+    """Algorithmic FLOPs and HBM bytes per launch of the force kernel, over D
+    monomials or, with nfun (FUNCTIONS), over that many functions in D's place.
 
     FLOPs, the per-atom work of the force step (everything after the MLP but
     the gather): per pair inside rc the U and V contractions 2 x (2 K D)
@@ -244,6 +253,7 @@ def algorithmic(cfg, npairs_rc, nlist, B, K, D, nin, form):
     (4 B/entry) and the pair force of every entry (16 B)."""
     n = cfg["natoms"]
     M = {1: 1, 4: 2, 10: 3, 20: 4}[D]
+    D = nfun or D
     flops = npairs_rc * (4.0 * K * D + 10.0 * K + (2 * K + 3) + (2 * D + 3) + 6.0 * D) \
         + n * B * (2 * M + 1) * D * K
     per_atom = 4 * B * K * D + 8 * nin + 48
@@ -333,8 +343,9 @@ def run_ours_sampled(args, rank, world, local, clk):
     npairs_rc = len(ent)
     nlist = len(sys_.neighbor_list(model.cutmax + 1.0)[1])
     B, K, D = model.nelt, model.num_filters, {1: 1, 2: 4, 3: 10, 4: 20}[model.mmax]
+    E = FUNCTIONS[D]
     flops, abytes = algorithmic(cfg, npairs_rc, nlist, B, K, D, model.n_desc,
-                                sys_.force_variant())
+                                sys_.force_variant(), nfun=E)
     fcnt, fms = prof["force"]
     force_ms = fms / max(fcnt, 1)
     hbm_peak, peak_kind = measured_peaks()
@@ -375,7 +386,7 @@ def run_ours_sampled(args, rank, world, local, clk):
         return {"ms": ms_, "bound": "fp32", "flops": fl, "achieved_tflops": tf,
                 "frac": tf / fp32_peak}
 
-    desc_flops = npairs_rc * (2.0 * K * D + 10.0 * K + D) + n * B * (2 * Minv + 1) * D * K
+    desc_flops = npairs_rc * (2.0 * K * E + 10.0 * K + E) + n * B * (2 * Minv + 1) * E * K
     # each pair force is read twice (as an atom's own and as its partner's)
     # but needs to leave HBM once
     gather_bytes = nlist * (16 + 4) + n * (24 + 4)
@@ -408,8 +419,8 @@ def run_ours_sampled(args, rank, world, local, clk):
                    "achieved_gbs": gather_bytes / (g_ms / 1000.0) / 1e9,
                    "frac": gather_bytes / (g_ms / 1000.0) / 1e9 / hbm_peak},
         "fp32_peak_tflops": fp32_peak,
-        "work": "descriptor: per pair inside rc P 2KD + radial 10K + monomials D, per atom "
-                "and block G (2M+1)DK; mlp: 2 x (forward + backward MACs) per atom; force: "
+        "work": "descriptor: per pair inside rc P 2KE + radial 10K + functions E (16 at rank "
+                "3), per atom and block G (2M+1)EK; mlp: 2 x (forward + backward MACs) per atom; force: "
                 "as roofline; gather: per list entry its pair force (16 B, read "
                 "once; the partner read is the same array) and partner slot (4 B), per atom "
                 "force (24 B) and row length",
@@ -1073,6 +1084,8 @@ def profile_step(args):
     s.set_atoms(x, t, v)
     if args.profile_desc:
         s.set_descriptor_variant(args.profile_desc)
+    if args.profile_force:
+        s.set_force_variant(args.profile_force)
     for _ in range(args.profile_step):
         s.compute(1, 1, 1.0)
     print(json.dumps({"profile_step": args.profile_step, "config": args.config,

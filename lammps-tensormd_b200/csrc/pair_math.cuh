@@ -315,10 +315,9 @@ __device__ inline void moments(float x, float y, float z, float M[D]) {
 // that feed them, and rows of 64 bytes.  The descriptor accumulates P over the
 // set {1, x, y, z, zz - c, xy, xz, xx - yy, yz, x (xx - s), x (yy - zz),
 // y (yy - s), y (zz - xx), z (zz - s), z (xx - yy), xyz}, orthogonal for c = 1/3
-// and s = 3/5: a
-// monomial's sum, put together again from orthogonal parts, carries the
-// rounding noise of its direct sum and no more (with xx - zz and the like,
-// sums over xyy came out 1.5 times as noisy).  The pair force evaluates Q(u)
+// and s = 3/5: a monomial's sum, put together again from orthogonal parts,
+// carries the rounding noise of its direct sum and no more (with xx - zz and the
+// like, sums over xyy came out 1.5 times as noisy).  The pair force evaluates Q(u)
 // with zz eliminated, over {1, x, y, z, xx, xy, xz, yy, yz, xxx, xxy, xxz,
 // xyy, xyz, yyy, yyz}.
 // c and s are the nearest numbers of 12 and 9 bits, so that the shares of P_0 and

@@ -24,6 +24,16 @@ def test_force_step_work_at_the_benchmark_shape():
     assert nbytes == n * (1280 + 512 + 48 + 4) + pairs * 48
 
 
+def test_force_step_work_over_the_functions_that_run():
+    """Rank 3 runs over 16 functions: per pair 4 x 256 + 160 + 35 + 35 + 96 FLOP,
+    per atom 9 x 256; P rows of 64 bytes."""
+    n, pairs, nlist = 128000, 9_750_000, 15_500_000
+    flops, nbytes = bench.algorithmic({"natoms": n}, pairs, nlist, 1, 16, 20, 64, "pair_lane8",
+                                      nfun=bench.FUNCTIONS[20])
+    assert flops == pytest.approx(pairs * (1024 + 160 + 35 + 35 + 96) + n * 9 * 256)
+    assert nbytes == n * (1024 + 512 + 48 + 4) + pairs * 48
+
+
 def test_whole_job_value_of_replicas():
     # 4 replicas of 1,000 atoms, 10 steps each, the slowest took 2 ms
     assert bench.replicas_value(1000, 10, 4, 2.0) == pytest.approx(2.0e7)
