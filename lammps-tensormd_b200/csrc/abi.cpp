@@ -178,6 +178,10 @@ int alloc_neighbors(tmd_system *s, int cap) {
   drop_graph(s);
   cap = (cap + 31) / 32 * 32;
   if (cap > 4096) return fail(TMD_ERR_CAPACITY, "more than 4096 neighbors per atom");
+  // from here to the end there are no rows, and so no atoms to compute
+  const bool had_atoms = s->have_atoms;
+  s->have_atoms = false;
+  s->cap = 0;
   dfree(s->tmp); dfree(s->nbr); dfree(s->rev); dfree(s->pdf); dfree(s->pgeo);
   size_t tot = (size_t)s->natoms_cap * cap;
   TMD_CUDA(dalloc(&s->tmp, tot));
@@ -187,6 +191,7 @@ int alloc_neighbors(tmd_system *s, int cap) {
   TMD_CUDA(dalloc(&s->pgeo, 2 * tot));
   s->cap = cap;
   s->capp = pow2_at_least(cap);
+  s->have_atoms = had_atoms;
   return TMD_OK;
 }
 
@@ -1348,15 +1353,14 @@ int tmd_system_set_atoms(tmd_system *s, int n, const double *x, const int *type,
     TMD_CUDA(cudaMemsetAsync(s->image, 0, 3 * n * sizeof(int), s->st));
   }
   TMD_CUDA(cudaStreamSynchronize(s->st));
-  s->have_atoms = true;
   s->forces_valid = false;
-  if (n == 0) return TMD_OK;
-  int cap = initial_cap(s);
+  const int cap = n > 0 ? initial_cap(s) : 0;
   if (cap > s->cap) {
     rc = alloc_neighbors(s, cap);
     if (rc) return rc;
   }
-  return rebuild_now(s);
+  s->have_atoms = true;
+  return n > 0 ? rebuild_now(s) : TMD_OK;
 }
 
 int tmd_system_set_atoms_ghost(tmd_system *s, int nlocal, int nghost, const double *x,
@@ -1401,18 +1405,17 @@ int tmd_system_set_atoms_ghost(tmd_system *s, int nlocal, int nghost, const doub
     TMD_CUDA(cudaMemsetAsync(s->image, 0, 3 * (size_t)n * sizeof(int), s->st));
   }
   TMD_CUDA(cudaStreamSynchronize(s->st));
-  s->have_atoms = true;
   s->forces_valid = false;
-  if (n == 0) return TMD_OK;
   // rows for the density inside the atoms' own bounding box
   double vol = 1.0;
   for (int a = 0; a < 3; a++) vol *= std::max(hi[a] - lo[a], 1.0);
-  const int cap = cap_for_density(s, n / vol);
+  const int cap = n > 0 ? cap_for_density(s, n / vol) : 0;
   if (cap > s->cap) {
     rc = alloc_neighbors(s, cap);
     if (rc) return rc;
   }
-  return rebuild_now(s);
+  s->have_atoms = true;
+  return n > 0 ? rebuild_now(s) : TMD_OK;
 }
 
 int tmd_system_set_positions(tmd_system *s, const double *x) {

@@ -5,7 +5,7 @@ when the atom count grows, the rows of the neighbor list being long enough."""
 import numpy as np
 import pytest
 
-from tmd_b200 import TensorMDModel, TensorMDSystem, synth
+from tmd_b200 import TensorMDModel, TensorMDSystem, TmdError, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +36,38 @@ def test_growing_atom_sets_allocate_nothing(tmp_path):
     for n in (500, 4000, 12000, len(x)):
         use(n)
     assert _free() == before
+
+
+@pytest.mark.parametrize("ghost", [False, True])
+def test_refused_atoms_leave_nothing_to_compute(tmp_path, ghost):
+    """set_atoms beyond 4,096 neighbors per atom is refused; the atoms of the call
+    before are gone by then, so a compute is refused too, until atoms are set."""
+    p = tmp_path / "m.npz"
+    syms = synth.gaussian_potential(p, nelt=1, num_filters=4, rc=6.0, max_moment=1, hidden=(16,),
+                                    actfn=2, seed=2)
+    s = TensorMDSystem(TensorMDModel(f"{p} {' '.join(syms)}"), 2500, 1.0)
+    x, t, box, _ = synth.build_system("fcc", 3.6, (4, 4, 4), sigma=0.05, nelt=1, seed=3)
+
+    def use(x, t):
+        if ghost:
+            s.set_atoms_ghost(len(x) // 2, x, t)
+        else:
+            s.set_atoms(x, t)
+
+    s.set_box(box)
+    use(x, t)
+    ref = s.compute(1, 1)
+    dense = np.random.default_rng(5).uniform(0.0, 8.0, (2500, 3))  # 5 atoms per A^3
+    if not ghost:
+        s.set_box(np.array([0, 0, 0, 8.0, 8.0, 8.0, 0, 0, 0]))
+    with pytest.raises(TmdError) as err:
+        use(dense, np.ones(2500, dtype=np.int32))
+    assert err.value.code == -4
+    with pytest.raises(TmdError) as err:
+        s.compute(1, 1)
+    assert "set_atoms" in str(err.value)
+    if not ghost:
+        s.set_box(box)
+    use(x, t)
+    again = s.compute(1, 1)
+    assert np.array_equal(again["f"], ref["f"]) and again["energy"] == ref["energy"]
