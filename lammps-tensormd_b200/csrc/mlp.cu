@@ -33,6 +33,9 @@ __global__ void k_mlp_activation(int actfn, int n, const float *__restrict__ z,
 
 // Column-block width of a net: the narrowest of 32, 64, 128 that holds its
 // widest hidden layer in one block (wider layers take several blocks of 128).
+// Widths between the blocks run padded, against the kernels this one replaced at
+// 128,000 atoms: 80-80-80 878 -> 458 us, 96-96 568 -> 324, 160-160 1131 -> 987,
+// 40-40 173 -> 109.
 int mlp_nt(int nl, const int *sizes) {
   int maxh = 1;
   for (int l = 1; l < nl; l++) maxh = std::max(maxh, sizes[l]);

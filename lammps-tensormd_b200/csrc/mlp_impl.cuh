@@ -31,7 +31,8 @@
 // sums bit for bit and before the activations below: 16 atoms of a 512-64x4 residual net 111 -> 40 us, 4,000
 // atoms 64-64-64 49 -> 14, 23,040 atoms 128-128x3 residual 270 -> 169, 128,000
 // atoms 64-64-64 180 -> 160, 432,000 atoms 512-128x3 5.86 -> 4.50 ms (56% of
-// the FP32 peak).  The producer needs a warp of its own: in a consumer warp
+// the FP32 peak).  (8 row registers at 128 columns spill 12 bytes, outside the
+// GEMM.)  The producer needs a warp of its own: in a consumer warp
 // its waits and copies hold up that warp's FMAs (5.1 ms).
 //
 // Sums per output run over the reduction index in ascending order whatever R

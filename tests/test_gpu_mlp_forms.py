@@ -1,11 +1,11 @@
 """FP32 MLP forms against the FP64 oracle on shapes the benchmark configs do
 not reach.
 
-The warp-tile form runs every MLP whose hidden layers are 64 wide and not
-residual: each activation kind, several elements (weights reloaded when a
-CTA's tiles change element), input widths that are not multiples of the
-64-column GEMM pass (dE/dG columns masked), one and three hidden layers.  The
-resident form runs the other widths and the residual MLPs.  Every case must
+One kernel runs them all, with blocks of 32, 64 or 128 columns and tiles by the
+atom count: each activation kind, several elements (biases and output weights
+reloaded when a CTA's tiles change element), input widths that are not multiples
+of the column block (dE/dG columns masked), one and three hidden layers, residual
+MLPs, widths between the blocks.  Every case must
 meet the plain-form bars (force relative RMS 1e-5, energy 5e-7 eV/atom, or
 2e-7 of the per-atom energy where residual layers make it large, virial
 1e-5)."""
