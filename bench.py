@@ -398,7 +398,9 @@ def run_ours_sampled(args, rank, world, local, clk):
     period = steps_all / max(rebuilds + prof_rebuilds, 1)
     sbytes = step_bytes_s8d(n, nlist, model.n_desc, period)
     step_traffic = 0
-    for kn in ("k_descriptor_w", "k_mlp_fp32", kname, "k_gather"):
+    desc_kernels = {"wide": ("k_descriptor_w",), "split": ("k_pair_geo", "k_descriptor_c"),
+                    "wide2": ("k_descriptor_w2",), "filter4": ("k_descriptor", "k_invariants")}
+    for kn in (*desc_kernels[sys_.descriptor_variant()], "k_mlp_fp32", kname, "k_gather"):
         tr = ncu_traffic(args.config, kn)
         step_traffic = None if (tr is None or step_traffic is None) else step_traffic + tr
     step_roofline = {
