@@ -370,10 +370,11 @@ int desc_form(const tmd_system *s) {
 
 int default_force_variant(const tmd_model *m) {
   // Whole pairs per lane, 8 lanes per atom up to 16 filters and 16 above (the
-  // staging of dE/dP per atom grows with K).  With 8 / 16 / 32 lanes inside a
-  // step on the B200: 16 Gaussians, 128,000 atoms 294 / 300 / 354 us; 32-filter
-  // table, 23,276 atoms 267 / 243 / 238, 432 atoms 50 / 27 / 15; 64-filter
-  // table, 23,276 atoms 684 / 477 / 484, 432 atoms 76 / 43 / 27.  The order of
+  // staging of dE/dP per atom grows with K).  With 8 / 16 / 32 lanes on the B200:
+  // 16 Gaussians, 128,000 atoms 299 / 300 / 354 us (each launch cold; back to
+  // back 288 / 285 / 341); inside a step, 32-filter table, 23,276 atoms 267 /
+  // 243 / 238, 432 atoms 50 / 27 / 15; 64-filter table, 23,276 atoms 684 / 477 /
+  // 484, 432 atoms 76 / 43 / 27.  The order of
   // the virial sum follows the lanes, so the choice goes by K alone and not by
   // the number of atoms: jobs of the server must not see each other.
   return m->kp.K <= 16 ? kForcePairLane8 : kForcePairLane16;
