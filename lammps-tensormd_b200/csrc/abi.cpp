@@ -158,11 +158,16 @@ int bin_setup(tmd_system *s) {
   b.ncell = (int)ncell;
   s->bin = b;
   if (b.ncell > s->ncell_alloc) {
+    // (a failed allocation leaves no bins, and so no atoms to compute)
+    const bool had_atoms = s->have_atoms;
+    s->have_atoms = false;
     dfree(s->cell_count); dfree(s->cell_start); dfree(s->cell_cursor);
+    s->ncell_alloc = 0;
     TMD_CUDA(dalloc(&s->cell_count, b.ncell));
     TMD_CUDA(dalloc(&s->cell_start, b.ncell + 1));
     TMD_CUDA(dalloc(&s->cell_cursor, b.ncell));
     s->ncell_alloc = b.ncell;
+    s->have_atoms = had_atoms;
   }
   return TMD_OK;
 }
@@ -533,6 +538,7 @@ int set_elements(tmd_system *s, int n, const int *elem) {
 int thermo_reserve(tmd_system *s, long count) {
   if (count > s->thermo_alloc) {
     dfree(s->thermo_d);
+    s->thermo_alloc = 0;
     TMD_CUDA(dalloc(&s->thermo_d, (size_t)count));
     s->thermo_alloc = count;
   }
@@ -541,8 +547,9 @@ int thermo_reserve(tmd_system *s, long count) {
 
 // Device checkpoint of the dynamic state for rolling back a chunk of steps.
 int checkpoint_reserve(tmd_system *s) {
-  if (!s->ck_x) {
+  if (!s->ck_img) {  // the last of them: all four are there
     const size_t N = s->natoms_cap;
+    dfree(s->ck_x); dfree(s->ck_v); dfree(s->ck_f);
     TMD_CUDA(dalloc(&s->ck_x, 3 * N));
     TMD_CUDA(dalloc(&s->ck_v, 3 * N));
     TMD_CUDA(dalloc(&s->ck_f, 3 * N));
@@ -550,6 +557,7 @@ int checkpoint_reserve(tmd_system *s) {
   }
   if (s->nhc_alloc > s->ck_nhc_alloc) {
     dfree(s->ck_nhc);
+    s->ck_nhc_alloc = 0;
     TMD_CUDA(dalloc(&s->ck_nhc, s->nhc_alloc));
     s->ck_nhc_alloc = s->nhc_alloc;
   }
@@ -586,6 +594,7 @@ int nhc_prepare(tmd_system *s, const NvtSpec &nvt, int nsteps, double dt) {
   if (G > s->nhc_alloc) {
     dfree(s->nhc);
     dfree(s->nhc_ke);
+    s->nhc_alloc = 0;
     TMD_CUDA(dalloc(&s->nhc, G));
     TMD_CUDA(dalloc(&s->nhc_ke, G));
     s->nhc_alloc = G;
